@@ -30,7 +30,6 @@ namespace {
 
 using namespace trav;
 
-
 template <bool COUNT>
 __device__ __forceinline__ void flush_counters(uint32_t err, uint32_t nvis, uint32_t ntri, uint32_t *err_out, unsigned long long *counters) {
     if (err) atomicOr(err_out, err);
@@ -120,17 +119,17 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
     Stack<DEEP, BLOCK, SDEPTH> st;
     st.smem = s_stack + threadIdx.x;
     st.sp = 0;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t lanemask_lt = (1u << lane) - 1u;
     uint32_t err = 0, nvis = 0, ntri = 0;
-    uint32_t ri = NO_RAY, mi = 0, visits = 0, steps = 0;
+    uint32_t ri = NO_RAY, mi = 0, visits = 0;
     uint32_t tstk[TLAS ? TLAS_STACK : 1]; // the ray's instance-tree stack (scenes with an instance tree)
     int tsp = 0;
     bool in_mesh = false;
-    Best best;
+    constexpr bool BEST_SMEM = (SDEPTH * 8 + 12) * BLOCK <= 48 * 1024;
+    __shared__ float s_best[BEST_SMEM ? 3 * BLOCK : 1];
+    LaneBest<BLOCK, BEST_SMEM> best;
     best.t = 0.0f;
-    best.u = best.v = 0.0f;
-    best.prim = best.obj = -1;
+    best.prim = -1;
+    if constexpr (BEST_SMEM) best.slot = s_best + threadIdx.x;
     LocalRay r = make_local_ray(0.0f, 0.0f, 0.0f, 1.0f, 1.0f, 1.0f);
     MeshRef mr{};
     uint32_t ng_base = 0, ng_bits = 0, tg_base = 0, tg_bits = 0;
@@ -139,13 +138,13 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
         // ---- refill lanes that have no ray
         const uint32_t need = __ballot_sync(0xffffffffu, ri == NO_RAY);
         if (!pool_empty && need != 0 && (__popc(need) >= refill_min || need == 0xffffffffu)) {
-            const uint32_t leader = __ffs(need) - 1;
+            const uint32_t leader = __ffs(need) - 1, lane = threadIdx.x & 31u;
             uint32_t base = 0;
             if (lane == leader) base = atomicAdd(next_ray, (uint32_t)__popc(need));
             base = __shfl_sync(0xffffffffu, base, leader);
             if (base + __popc(need) >= n) pool_empty = true;
             if (ri == NO_RAY) {
-                const uint32_t idx = base + __popc(need & lanemask_lt);
+                const uint32_t idx = base + __popc(need & ((1u << lane) - 1u));
                 if (idx < n) {
                     ri = order ? __ldg(order + idx) : idx;
                     mi = 0;
@@ -155,19 +154,17 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
                     }
                     in_mesh = false;
                     best.t = __ldg(&rays[2ull * ri].w);
-                    best.u = best.v = 0.0f;
-                    best.prim = best.obj = -1;
+                    best.prim = -1;
                 }
             }
         }
         if (pool_empty && __all_sync(0xffffffffu, ri == NO_RAY)) break;
-        // A lane without work this iteration falls through to the next one;
-        // with ONE the warp meets again (__syncwarp) after each phase, which
-        // keeps lanes that took different branches from drifting into
-        // different iterations (measured: 4.28 ms without, 3.7 ms with, per
-        // 4M-ray launch of the microbench on B200)
+        // A lane without work this iteration falls through to the next one, the
+        // warp meeting again (__syncwarp) after each phase, which keeps lanes
+        // that took different branches from drifting into different iterations
+        // (one triangle per step, 4M-ray launch of the microbench on B200:
+        // 4.28 ms without, 3.7 ms with)
         bool idle = ri == NO_RAY;
-        if (!ONE && idle) continue;
         // ---- next instance whose box the ray enters, or the end of the ray
         // (a ray whose scene has no instance left is done without reading it
         // again; a multi-scene ray reads its scene view first)
@@ -189,11 +186,10 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
                     mr = mesh_of(lsv, ir, m);
                     r = transform_ray(ir, r0, r1);
                     ng_base = 0;
-                    ng_bits = (1u << (24 + r.oct)) | 1u;
+                    ng_bits = r.root_bits();
                     tg_bits = 0;
                     st.sp = 0;
                     visits = 0;
-                    steps = 0;
                     in_mesh = true;
                 }
             }
@@ -210,54 +206,40 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
                 mr = mesh_of(lsv, ir, (int)mi - 1);
                 r = transform_ray(ir, r0, r1);
                 ng_base = 0;
-                ng_bits = (1u << (24 + r.oct)) | 1u;
+                ng_bits = r.root_bits();
                 tg_bits = 0;
                 st.sp = 0;
                 visits = 0;
-                steps = 0;
                 in_mesh = true;
                 break;
             }
           }
             if (!in_mesh) {
-                const float4 h = make_float4(__int_as_float(best.prim), best.t, best.prim >= 0 ? best.u : 0.0f, best.prim >= 0 ? best.v : 0.0f);
+                const bool found = best.prim >= 0;
+                const float4 h = make_float4(__int_as_float(best.prim), best.t, found ? best.u() : 0.0f, found ? best.v() : 0.0f);
                 if (stream_hint) __stcs(hits + ri, h);
                 else hits[ri] = h;
-                if (obj_out) obj_out[ri] = best.obj;
+                if (obj_out) obj_out[ri] = found ? best.obj() : -1;
                 ri = NO_RAY;
                 idle = true;
-                if (!ONE) continue;
             }
         }
-        if (ONE) __syncwarp();
-        // ---- one traversal step: a node visit and the triangles it hits. A
-        // mesh takes at most node_count steps; more means a corrupt structure.
-        // Every group pushed today has a node bit, so the else branch (a group
-        // of triangles only, tested as such) does not run; keeping the node
-        // step under this test measured 4.8 ms instead of 6.9 ms per 4M-ray
-        // launch on B200, the compiler keeping the warp converged around it.
-        if (!idle && (!ONE || tg_bits == 0)) {
-            bool ok = ++steps <= mr.node_count + 8u;
-            if (!ok) err |= TRACE_ERR_LIMIT;
-            if (ok && ng_bits > 0x00FFFFFFu) {
-                ok = node_step<COUNT>(mr, r, best.t, ng_base, ng_bits, tg_base, tg_bits, st, visits, err, nvis);
-            } else if (ok) {
-                tg_base = ng_base;
-                tg_bits = ng_bits;
-                ng_bits = 0;
-            }
-            if (!ok) {
+        __syncwarp();
+        // ---- a node visit (the node step bounds a mesh's visits by its node
+        // count) for the lanes whose last node's triangles are done
+        if (!idle && tg_bits == 0) {
+            if (!node_step<COUNT>(mr, r, best.t, ng_base, ng_bits, tg_base, tg_bits, st, visits, err, nvis)) {
                 in_mesh = false;
                 mi = 0xffffffffu; // abandon the ray; the error flag reports it
                 tsp = 0;
                 tg_bits = 0;
                 idle = true;
-                if (!ONE) continue;
             }
         }
-        if (ONE) __syncwarp();
+        __syncwarp();
+        // ---- triangles: one per lane, then (not with ONE) the others
         bool stop = false;
-        if (ONE) {
+        while (true) {
             if (!idle && tg_bits) {
                 const uint32_t k = __ffs(tg_bits) - 1;
                 tg_bits &= tg_bits - 1;
@@ -270,21 +252,9 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
                     tri_test<COUNT>(mr, r, tg_base + k, best, err, ntri);
                 }
             }
-        } else {
-            while (!idle && tg_bits) {
-                const uint32_t k = __ffs(tg_bits) - 1;
-                tg_bits &= tg_bits - 1;
-                if (ANY) {
-                    if (tri_test<COUNT, true>(mr, r, tg_base + k, best, err, ntri)) {
-                        stop = true;
-                        tg_bits = 0;
-                    }
-                } else {
-                    tri_test<COUNT>(mr, r, tg_base + k, best, err, ntri);
-                }
-            }
+            if (ONE || !__any_sync(0xffffffffu, !idle && tg_bits)) break;
         }
-        if (ONE) __syncwarp();
+        __syncwarp();
         if (idle) continue;
         if (ANY && stop) { // a solid triangle blocks the ray: no further instance
             in_mesh = false;

@@ -25,9 +25,33 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
     return r;
 }
 
-// Byte k of word as the float 1 + byte * 2^-15 (0x3F80bb00): exact, one permute.
-__device__ __forceinline__ float byte_to_unit(uint32_t word, uint32_t k) {
-    return __uint_as_float(__byte_perm(word, 0x3F800000u, 0x7604u | (k << 4)));
+// Byte k of word as the float 2^15 + byte (0x4700bb00): exact, one permute.
+__device__ __forceinline__ float byte_to_float(uint32_t word, uint32_t k) {
+    return __uint_as_float(__byte_perm(word, 0x47000000u, 0x7604u | (k << 4)));
+}
+
+// Pairs of floats in one 64-bit register and their packed arithmetic
+// (sm_100): each half is rounded as the scalar operation rounds it.
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
 // The reference's slab test, exactly (bbox_test, CoreRef.cpp:64-86).
@@ -79,12 +103,61 @@ __device__ __forceinline__ float safe_inv(float v) {
 struct Best {
     float t, u, v;
     int prim, obj;
+    __device__ __forceinline__ void rest(float u_, float v_, int obj_) {
+        u = u_;
+        v = v_;
+        obj = obj_;
+    }
+};
+
+// The best hit of a lane of the persistent kernel: what the tests compare
+// stays in registers; u, v and the instance, written on an accepted hit and
+// read when the ray ends, are in shared memory (word k of this thread at
+// slot[k * STRIDE]). Three registers less keep the 64-register instance
+// of the kernel from spilling.
+// IN_SMEM false (block shapes whose stack fills the static shared memory):
+// everything in registers.
+template <int STRIDE, bool IN_SMEM>
+struct LaneBest;
+
+template <int STRIDE>
+struct LaneBest<STRIDE, false> {
+    float t;
+    int prim;
+    float bu, bv;
+    int bobj;
+    __device__ __forceinline__ void rest(float u, float v, int obj) {
+        bu = u;
+        bv = v;
+        bobj = obj;
+    }
+    __device__ __forceinline__ float u() const { return bu; }
+    __device__ __forceinline__ float v() const { return bv; }
+    __device__ __forceinline__ int obj() const { return bobj; }
+};
+
+template <int STRIDE>
+struct LaneBest<STRIDE, true> {
+    float t;
+    int prim;
+    float *slot;
+    __device__ __forceinline__ void rest(float u, float v, int obj) {
+        slot[0] = u;
+        slot[STRIDE] = v;
+        slot[2 * STRIDE] = __int_as_float(obj);
+    }
+    __device__ __forceinline__ float u() const { return slot[0]; }
+    __device__ __forceinline__ float v() const { return slot[STRIDE]; }
+    __device__ __forceinline__ int obj() const { return __float_as_int(slot[2 * STRIDE]); }
 };
 
 // Ray in the space of the instance being traversed.
 struct LocalRay {
     float ox, oy, oz, dx, dy, dz, ix, iy, iz;
-    uint32_t oct; // bit a set: direction negative on axis a
+    // bit a (0..2) set: the direction is negative on axis a; bit 3 + a set: it
+    // is zero there (the node step tests that axis by containment)
+    uint32_t oct;
+    __device__ __forceinline__ uint32_t root_bits() const { return (1u << (24 + (oct & 7u))) | 1u; } // the root as slot 0 of a virtual parent
 };
 
 struct MeshRef {
@@ -144,6 +217,7 @@ __device__ __forceinline__ LocalRay make_local_ray(float ox, float oy, float oz,
     r.iy = __frcp_rn(dy);
     r.iz = __frcp_rn(dz);
     r.oct = (r.ix < 0.0f ? 1u : 0u) | (r.iy < 0.0f ? 2u : 0u) | (r.iz < 0.0f ? 4u : 0u);
+    if (dx == 0.0f || dy == 0.0f || dz == 0.0f) r.oct |= (dx == 0.0f ? 8u : 0u) | (dy == 0.0f ? 16u : 0u) | (dz == 0.0f ? 32u : 0u);
     return r;
 }
 
@@ -227,6 +301,29 @@ __device__ __forceinline__ int tlas_next(const SceneView &sv, float4 r0, float s
     return -1;
 }
 
+// Children of a node whose slab on every zero axis of the ray (oct bits 3..5)
+// holds the ray's origin: on such an axis the ray never leaves its origin's
+// coordinate, so a box that does not span it is missed at every t. The decoded
+// planes p + q 2^e are exact floats (the product and sum below round nothing)
+// and lie a quantum outside the child's triangles, so no triangle whose box
+// spans the origin is dropped. Bytes are read again from the node: this runs
+// for rays that are parallel to an axis plane only.
+__device__ __forceinline__ uint32_t zero_axis_children(const WideNode *nd, uint32_t oct, float ox, float oy, float oz) {
+    uint32_t keep = 0xFFu;
+#pragma unroll 1
+    for (int a = 0; a < 3; a++) {
+        if (!((oct >> (3 + a)) & 1u)) continue;
+        const float o = a == 0 ? ox : (a == 1 ? oy : oz);
+        const float p = __ldg(&nd->p[a]), sc = __uint_as_float((uint32_t)__ldg(&nd->e[a]) << 23);
+#pragma unroll 1
+        for (int c = 0; c < 8; c++) {
+            const float lo = __fmaf_rn((float)__ldg(&nd->qlo[a][c]), sc, p), hi = __fmaf_rn((float)__ldg(&nd->qhi[a][c]), sc, p);
+            if (o < lo || o > hi) keep &= ~(1u << c); // (a NaN origin keeps every child)
+        }
+    }
+    return keep;
+}
+
 // Node step: takes the next child of node group (ng_base, ng_bits), tests
 // its 8 children and returns their hits as a node group (internal children,
 // bits 24..31, with the node's imask in bits 0..7) and a triangle group
@@ -237,7 +334,7 @@ __device__ __forceinline__ bool node_step(const MeshRef &mr, const LocalRay &r, 
                                           uint32_t &nvis) {
     const uint32_t j = __ffs(ng_bits >> 24) - 1;
     ng_bits &= ~(1u << (24 + j));
-    const uint32_t s = j ^ r.oct;
+    const uint32_t s = (j ^ r.oct) & 7u;
     const uint32_t ni = ng_base + __popc((ng_bits & 0xFFu) & ((1u << s) - 1u));
     if (ng_bits > 0x00FFFFFFu && !st.push(make_uint2(ng_base, ng_bits))) {
         err |= TRACE_ERR_STACK;
@@ -249,36 +346,48 @@ __device__ __forceinline__ bool node_step(const MeshRef &mr, const LocalRay &r, 
         err |= (ni >= mr.node_count) ? TRACE_ERR_BOUNDS : TRACE_ERR_LIMIT;
         return false;
     }
+    // a zero direction component leaves its axis' planes NaN, that is unbounded:
+    // without this a ray parallel to an axis plane entered every node its
+    // other two axes allow, thousands of them, and one such ray among the 4M of
+    // a launch decided the launch's time (5.4 to 14 ms against 3.2 ms on B200)
+    const uint32_t keep = r.oct > 7u ? zero_axis_children(mr.nodes + ni, r.oct, r.ox, r.oy, r.oz) : 0xFFu;
     const uint4 *np = reinterpret_cast<const uint4 *>(mr.nodes + ni);
     const uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
     if (COUNT) nvis++;
     const uint32_t imask = w0.w >> 24;
     // Slab parameter of plane q on one axis: t(q) = q * A + B with
     // A = 2^e * inv_d (exact: a power-of-two scaling) and B = (p - o) * inv_d.
-    // It is evaluated as one FMA on the byte read as the float
-    // v = 1 + q * 2^-15: t = v * (2^15 A) + (B - 2^15 A), where 2^15 A is
-    // exact and v * 2^15 A = 2^15 A + q A exactly inside the FMA. Rounding
+    // It is evaluated as one FMA on the byte read as the float v = 2^15 + q:
+    // t = v * A + (B - 2^15 A), v * A exact inside the FMA. Rounding
     // B - 2^15 A, then -/+ slack, then the FMA's result errs by less than
     // 3u(|B| + 33024|A|) (u = 2^-24); the slack 2^-21 (|B| + 33024|A|)
     // moves the near planes down and the far planes up by more than that,
     // so the test accepts every box that the exact slab test on the decoded
     // box accepts. (An overflowing 2^15 A gives NaN planes: that axis is
     // left unbounded, still conservative.)
-    float A[3], Bn[3], Bf[3];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const float p = __uint_as_float(a == 0 ? w0.x : (a == 1 ? w0.y : w0.z));
-        const float sc = __uint_as_float(((w0.w >> (8 * a)) & 0xFFu) << 23);
-        const float inv = a == 0 ? r.ix : (a == 1 ? r.iy : r.iz);
-        const float o = a == 0 ? r.ox : (a == 1 ? r.oy : r.oz);
-        const float Aa = __fmul_rn(sc, inv);
-        const float B = __fmul_rn(__fsub_rn(p, o), inv);
-        const float slack = __fmul_rn(__fmaf_rn(fabsf(Aa), 33024.0f, fabsf(B)), 4.76837158203125e-07f);
-        const float B0 = __fmaf_rn(-32768.0f, Aa, B);
-        A[a] = __fmul_rn(Aa, 32768.0f);
-        Bn[a] = __fsub_rn(B0, slack);
-        Bf[a] = __fadd_rn(B0, slack);
-    }
+    // The step is bound by instruction issue. The set-up of the x and y axes
+    // goes through packed arithmetic; the children's FMAs stay scalar, packed
+    // ones measured slower (the pairs' registers spill at 64 a thread: 3.41
+    // against 3.18 ms per 4M-ray launch; at 72 a thread 3.26).
+    const float scx = __uint_as_float((w0.w & 0xFFu) << 23), scy = __uint_as_float(((w0.w >> 8) & 0xFFu) << 23),
+                scz = __uint_as_float(((w0.w >> 16) & 0xFFu) << 23);
+    const unsigned long long ixy = pack2(r.ix, r.iy);
+    const unsigned long long Axy = mul2(pack2(scx, scy), ixy);
+    const unsigned long long Bxy = mul2(add2(pack2(__uint_as_float(w0.x), __uint_as_float(w0.y)), pack2(-r.ox, -r.oy)), ixy);
+    float Ax, Ay, Bx, By;
+    unpack2(Axy, Ax, Ay);
+    unpack2(Bxy, Bx, By);
+    const float Az = __fmul_rn(scz, r.iz), Bz = __fmul_rn(__fsub_rn(__uint_as_float(w0.z), r.oz), r.iz);
+    const unsigned long long Sxy = pack2(__fmaf_rn(fabsf(Ax), 33024.0f, fabsf(Bx)), __fmaf_rn(fabsf(Ay), 33024.0f, fabsf(By)));
+    const float Sz = __fmaf_rn(fabsf(Az), 33024.0f, fabsf(Bz));
+    const unsigned long long B0xy = fma2(Axy, pack2(-32768.0f, -32768.0f), Bxy);
+    const float B0z = __fmaf_rn(-32768.0f, Az, Bz);
+    constexpr float SLACK = 4.76837158203125e-07f; // 2^-21
+    const unsigned long long Bnxy = fma2(Sxy, pack2(-SLACK, -SLACK), B0xy), Bfxy = fma2(Sxy, pack2(SLACK, SLACK), B0xy);
+    const float Bnz = __fmaf_rn(Sz, -SLACK, B0z), Bfz = __fmaf_rn(Sz, SLACK, B0z);
+    float Bnx, Bny, Bfx, Bfy;
+    unpack2(Bnxy, Bnx, Bny);
+    unpack2(Bfxy, Bfx, Bfy);
     // Near/far plane words by direction sign, so that a NaN slab value
     // (origin on a plane of a box the ray runs parallel to) leaves that axis
     // unbounded, which keeps the test conservative. Planes: lo x = w2.xy,
@@ -287,22 +396,21 @@ __device__ __forceinline__ bool node_step(const MeshRef &mr, const LocalRay &r, 
     const uint32_t nxa = nx ? w3.z : w2.x, nxb = nx ? w3.w : w2.y, fxa = nx ? w2.x : w3.z, fxb = nx ? w2.y : w3.w;
     const uint32_t nya = ny ? w4.x : w2.z, nyb = ny ? w4.y : w2.w, fya = ny ? w2.z : w4.x, fyb = ny ? w2.w : w4.y;
     const uint32_t nza = nz ? w4.z : w3.x, nzb = nz ? w4.w : w3.y, fza = nz ? w3.x : w4.z, fzb = nz ? w3.y : w4.w;
-    uint32_t hit8 = 0; // slots whose box the ray enters
+    uint32_t miss = 0; // sign bits of (far - near) shifted in, the last slot first: slots whose box the ray misses
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
+    for (int c = 7; c >= 0; c--) {
         const uint32_t k = (uint32_t)(c & 3);
-        const float tnx = __fmaf_rn(byte_to_unit(c < 4 ? nxa : nxb, k), A[0], Bn[0]);
-        const float tfx = __fmaf_rn(byte_to_unit(c < 4 ? fxa : fxb, k), A[0], Bf[0]);
-        const float tny = __fmaf_rn(byte_to_unit(c < 4 ? nya : nyb, k), A[1], Bn[1]);
-        const float tfy = __fmaf_rn(byte_to_unit(c < 4 ? fya : fyb, k), A[1], Bf[1]);
-        const float tnz = __fmaf_rn(byte_to_unit(c < 4 ? nza : nzb, k), A[2], Bn[2]);
-        const float tfz = __fmaf_rn(byte_to_unit(c < 4 ? fza : fzb, k), A[2], Bf[2]);
+        const float tnx = __fmaf_rn(byte_to_float(c < 4 ? nxa : nxb, k), Ax, Bnx), tfx = __fmaf_rn(byte_to_float(c < 4 ? fxa : fxb, k), Ax, Bfx);
+        const float tny = __fmaf_rn(byte_to_float(c < 4 ? nya : nyb, k), Ay, Bny), tfy = __fmaf_rn(byte_to_float(c < 4 ? fya : fyb, k), Ay, Bfy);
+        const float tnz = __fmaf_rn(byte_to_float(c < 4 ? nza : nzb, k), Az, Bnz), tfz = __fmaf_rn(byte_to_float(c < 4 ? fza : fzb, k), Az, Bfz);
         // [max(near planes, 0), min(far planes, best_t)] non-empty: the slab
-        // test with the ray's interval folded in (best_t >= 0)
+        // test with the ray's interval folded in (best_t >= 0); the difference
+        // is never negative when it is (inf - inf gives NaN, sign clear)
         const float tmin = max3f(tnx, tny, fmaxf(tnz, 0.0f));
         const float tmax = min3f(tfx, tfy, fminf(tfz, best_t));
-        if (tmin <= tmax) hit8 |= 1u << c;
+        miss = __funnelshift_l(__float_as_uint(__fsub_rn(tmax, tmin)), miss, 1);
     }
+    uint32_t hit8 = ~miss & keep;
     // internal children: bit 24 + (slot ^ octant), so that the node group
     // is taken in the ray's octant order
     uint32_t inner = hit8 & imask;
@@ -351,8 +459,8 @@ __device__ __forceinline__ bool tri_core(const float4 &t0, const float4 &t1, con
 // One triangle test; updates best when it is the closer hit. With SOLID,
 // returns whether that hit is on a solid triangle (TRI_SOLID_BIT), which ends
 // a shadow ray's search (IntersectTris_AnyHit, CoreRef.cpp:804-829).
-template <bool COUNT, bool SOLID = false>
-__device__ __forceinline__ bool tri_test(const MeshRef &mr, const LocalRay &r, uint32_t li, Best &best, uint32_t &err, uint32_t &ntri) {
+template <bool COUNT, bool SOLID = false, typename BEST>
+__device__ __forceinline__ bool tri_test(const MeshRef &mr, const LocalRay &r, uint32_t li, BEST &best, uint32_t &err, uint32_t &ntri) {
     if (li >= mr.tri_count) {
         err |= TRACE_ERR_BOUNDS;
         return false;
@@ -366,10 +474,8 @@ __device__ __forceinline__ bool tri_test(const MeshRef &mr, const LocalRay &r, u
         const int gp = (int)(mr.prim_base + __float_as_uint(t2.z));
         if (t > 0.0f && (t < best.t || (t == best.t && best.prim >= 0 && gp < best.prim))) {
             best.t = t;
-            best.u = __fmul_rn(detu, rdet);
-            best.v = __fmul_rn(detv, rdet);
             best.prim = gp;
-            best.obj = mr.obj;
+            best.rest(__fmul_rn(detu, rdet), __fmul_rn(detv, rdet), mr.obj);
             if (SOLID) return (__float_as_int(t1.y) & TRI_SOLID_BIT) != 0;
         }
     }
@@ -382,7 +488,7 @@ __device__ __forceinline__ bool tri_test(const MeshRef &mr, const LocalRay &r, u
 template <bool COUNT, typename ST>
 __device__ __forceinline__ void trace_mesh(const MeshRef &mr, const LocalRay &r, Best &best, ST &st, uint32_t &err,
                                            uint32_t &nvis, uint32_t &ntri) {
-    uint32_t ng_base = 0, ng_bits = (1u << (24 + r.oct)) | 1u; // the root as slot 0 of a virtual parent
+    uint32_t ng_base = 0, ng_bits = r.root_bits();
     uint32_t tg_base = 0, tg_bits = 0, visits = 0;
     st.sp = 0;
     while (true) {
@@ -406,7 +512,7 @@ __device__ __forceinline__ void trace_mesh(const MeshRef &mr, const LocalRay &r,
 // hit on a solid triangle. Returns true when it stopped there.
 template <typename ST>
 __device__ __forceinline__ bool trace_mesh_any(const MeshRef &mr, const LocalRay &r, Best &best, ST &st, uint32_t &err) {
-    uint32_t ng_base = 0, ng_bits = (1u << (24 + r.oct)) | 1u;
+    uint32_t ng_base = 0, ng_bits = r.root_bits();
     uint32_t tg_base = 0, tg_bits = 0, visits = 0, nvis = 0, ntri = 0;
     st.sp = 0;
     while (true) {
