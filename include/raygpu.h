@@ -304,7 +304,7 @@ int ray_scene_last_trace_info(ray_scene *s, ray_trace_info *out);
  * context's persisting-L2 limit, which lasts as long as the context).
  * instance_tree: 0 = traces walk an instance tree (a BVH over the instances'
  * world boxes, built on the GPU at commit, refitted when only transforms
- * changed; the reference's macro tree, SceneRef.cpp:492-516) from 32
+ * changed; the reference's macro tree, SceneRef.cpp:492-516) from 8
  * instances on and test the instance boxes in turn below that; 1 = the tree
  * from 2 instances on; -1 = never. */
 typedef struct ray_trace_tuning {

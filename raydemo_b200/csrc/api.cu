@@ -1259,7 +1259,7 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
         RG_CUDA_TRY(cudaStreamWaitEvent(other, s->pipe_ev[0], 0));
     }
     SceneView sv{static_cast<const WideNode *>(s->d_nodes.p), static_cast<const TriRec *>(s->d_leaf.p),
-                 static_cast<const InstanceRec *>(s->d_inst.p), s->n_inst_dev, s->tlas.nodes};
+                 static_cast<const InstanceRec *>(s->d_inst.p), s->n_inst_dev, s->tlas.nodes, s->tlas.order, s->tlas.count};
     RG_CUDA_TRY(s->d_next_ray.ensure(8)); // a work counter for each of two concurrent traces
     TraceParams tp;
     tp.persistent = s->tuning.kernel >= 2;
@@ -1294,6 +1294,7 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
         }
     }
     for (const MeshRec &m : s->meshes) tp.max_depth = std::max(tp.max_depth, m.bvh.depth);
+    if (s->tlas.nodes) tp.max_depth += tlas_stack_levels(s->tlas.depth());
     if (s->tuning.deep_stack) tp.max_depth = 0xffffffffu;
     uint32_t *next_ray = static_cast<uint32_t *>(s->d_next_ray.p);
     // reordered traces: the hash grid of SortRays_CPU over the scene's box (RendererRef.cpp:48-77)

@@ -1,6 +1,8 @@
 // GPU BVH construction for one mesh.
 #pragma once
 
+#include <vector>
+
 #include "common.cuh"
 
 namespace rg {
@@ -29,18 +31,24 @@ cudaError_t launch_preprocess_tris(const float *verts, const uint32_t *mat, uint
 int build_mesh_bvh(const TriRec *tris_ref, const float *aabb, uint32_t n, MeshBvh &out, cudaStream_t st);
 
 // The instance tree: an LBVH over the instances' world boxes (Morton codes
-// of the box centres, the same radix sort and binary radix tree as a mesh's
-// build), its node boxes computed bottom-up and packed into TlasNode
-// records. A refit keeps the topology and recomputes only the boxes (after
-// instances moved); a build is needed when the instance count changed.
+// of the box centres, the same radix sort, binary radix tree and collapse as
+// a mesh's build) as wide nodes with one instance per leaf slot, so that the
+// traversal tests it with the mesh nodes' own step (1,024 instances, 262,144
+// rays on B200: 0.84 ms; a binary tree of float boxes with its own stack in
+// local memory took 1.86). slot_src keeps what each
+// slot of a node holds; a refit (after instances moved) recomputes the boxes
+// over the same topology, a level of nodes per launch from the deepest up. A
+// build is needed when the instance count changed.
 struct InstTree {
     uint32_t n = 0;              // instances of the current topology (0: none built)
     float *aabb = nullptr;       // 6 floats per instance: world box
-    uint32_t *sorted = nullptr;  // sorted position -> instance index
-    uint32_t *left = nullptr, *right = nullptr, *parent = nullptr, *first = nullptr, *last = nullptr;
-    float *nb = nullptr;         // node boxes (6 floats per internal node)
-    uint32_t *flags = nullptr;   // arrival counters of the bottom-up passes
-    TlasNode *nodes = nullptr;   // n - 1 packed nodes
+    uint32_t *order = nullptr;   // leaf entry -> instance index
+    WideNode *nodes = nullptr;   // node 0 is the root; a level's nodes are contiguous
+    uint32_t *slot_src = nullptr; // 8 per node: INST_LEAF | instance, child node, or INST_EMPTY
+    float *box = nullptr;        // 6 floats per node
+    uint32_t count = 0;          // nodes
+    std::vector<uint32_t> level; // first node of each level, then the node count
+    uint32_t depth() const { return level.empty() ? 0u : (uint32_t)level.size() - 1u; }
 };
 void free_inst_tree(InstTree &t);
 // boxes: n world boxes (6 floats each) in host memory. refit: keep the

@@ -32,6 +32,8 @@ namespace rg {
 namespace {
 
 constexpr uint32_t LEAF = 0x80000000u;
+// InstTree::slot_src: an instance, or nothing; else a node
+constexpr uint32_t INST_LEAF = 0x80000000u, INST_EMPTY = 0xffffffffu;
 
 __device__ __forceinline__ float comp(const float3 &v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
 
@@ -227,28 +229,6 @@ __global__ void k_bottom_up(const float *__restrict__ aabb, const uint32_t *__re
     }
 }
 
-// Instance tree nodes from the binary radix tree and its node boxes: both
-// children's boxes (an instance's world box, or the child node's box) and
-// ids (TLAS_LEAF | instance index, or the node index).
-__global__ void k_tlas_pack(const float *__restrict__ aabb, const uint32_t *__restrict__ sorted, int n, const uint32_t *__restrict__ left,
-                            const uint32_t *__restrict__ right, const float *__restrict__ nb, TlasNode *__restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n - 1) return;
-    TlasNode t;
-    for (int c = 0; c < 2; c++) {
-        const uint32_t id = c == 0 ? left[i] : right[i];
-        float lo[3], hi[3];
-        child_box(id, aabb, sorted, nb, lo, hi);
-        for (int k = 0; k < 3; k++) {
-            t.lo[c][k] = lo[k];
-            t.hi[c][k] = hi[k];
-        }
-        t.child[c] = (id & LEAF) ? (TLAS_LEAF | sorted[id & ~LEAF]) : id;
-    }
-    t.pad[0] = t.pad[1] = 0;
-    out[i] = t;
-}
-
 // SAH weights of the cost programme: a wide node's box test and fetch, and one triangle test.
 constexpr float SAH_NODE = 1.0f, SAH_TRI = 1.2f;
 
@@ -275,6 +255,8 @@ __device__ __forceinline__ float slot_cost(uint32_t c, int j, const float *__res
 // of one slot and the best split of the j slots between the two children
 // (dec = the left child's share, 0 for one slot). open_k: the best split of
 // 8 slots when the node is opened as a wide node.
+// LEAF_MAX: triangles (or instances) a leaf slot holds at most.
+template <uint32_t LEAF_MAX>
 __global__ void k_wide_cost(const float *__restrict__ aabb, const uint32_t *__restrict__ sorted, int n, const uint32_t *__restrict__ left,
                             const uint32_t *__restrict__ right, const uint32_t *__restrict__ parent, const uint32_t *__restrict__ first,
                             const uint32_t *__restrict__ last, const float *__restrict__ nb, uint32_t *flags, float *cost,
@@ -314,7 +296,7 @@ __global__ void k_wide_cost(const float *__restrict__ aabb, const uint32_t *__re
             dist[j] = best;
             dk[j] = bk;
         }
-        const bool as_leaf = cnt <= (uint32_t)LEAF_MAX_TRIS;
+        const bool as_leaf = cnt <= LEAF_MAX;
         const float c1 = as_leaf ? area * (float)cnt * SAH_TRI : area * SAH_NODE + dist[8];
         __stcg(cost + 8ull * node, c1);
         dec[8ull * node] = as_leaf ? 0 : 1;
@@ -337,30 +319,23 @@ __device__ __forceinline__ uint32_t bin_count(uint32_t c, const uint32_t *first,
     return (c & LEAF) ? 1u : (last[c] - first[c] + 1u);
 }
 
-__global__ void k_collapse(const QItem *__restrict__ in, uint32_t n_in, QItem *__restrict__ out, uint32_t *__restrict__ counters,
-                           const float *__restrict__ aabb, const uint32_t *__restrict__ sorted, const TriRec *__restrict__ tris_ref,
-                           const uint32_t *__restrict__ left, const uint32_t *__restrict__ right, const uint32_t *__restrict__ first,
-                           const uint32_t *__restrict__ last, const float *__restrict__ nb, const uint8_t *__restrict__ dec,
-                           const uint8_t *__restrict__ open_k, WideNode *__restrict__ nodes, TriRec *__restrict__ leaf_tris) {
-    // counters: [0] wide nodes allocated, [1] leaf triangles allocated,
-    //           [2] items written to `out`, [3] maximum depth
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_in) return;
-    const QItem it = in[t];
-    uint32_t c[8];
+// The slots the cost programme chose for binary node `bin` (a sorted leaf:
+// itself alone): ids into c, returns how many.
+__device__ __forceinline__ int chosen_slots(uint32_t bin, const uint32_t *__restrict__ left, const uint32_t *__restrict__ right,
+                                            const uint8_t *__restrict__ dec, const uint8_t *__restrict__ open_k, uint32_t c[8]) {
     int nc;
-    if (it.bin & LEAF) {
-        c[0] = it.bin;
+    if (bin & LEAF) {
+        c[0] = bin;
         nc = 1;
     } else {
-        // the slots the cost programme chose: open it.bin into 8 slots, then
+        // the slots the cost programme chose: open bin into 8 slots, then
         // follow each subtree's choice for its share of them
         uint32_t sn[16];
         int sj[16], sp = 0;
-        const int k0 = min(max((int)open_k[it.bin], 1), 7);
-        sn[sp] = right[it.bin];
+        const int k0 = min(max((int)open_k[bin], 1), 7);
+        sn[sp] = right[bin];
         sj[sp++] = 8 - k0;
-        sn[sp] = left[it.bin];
+        sn[sp] = left[bin];
         sj[sp++] = k0;
         nc = 0;
         while (sp > 0 && nc < 8) {
@@ -378,18 +353,14 @@ __global__ void k_collapse(const QItem *__restrict__ in, uint32_t n_in, QItem *_
             }
         }
     }
-    float clo[8][3], chi[8][3];
-    float nlo[3] = {INFINITY, INFINITY, INFINITY}, nhi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int k = 0; k < nc; k++) {
-        child_box(c[k], aabb, sorted, nb, clo[k], chi[k]);
-        for (int a = 0; a < 3; a++) {
-            nlo[a] = fminf(nlo[a], clo[k][a]);
-            nhi[a] = fmaxf(nhi[a], chi[k][a]);
-        }
-    }
-    // octant slot assignment: slot bit a set <=> child lies on the high side of axis a
+    return nc;
+}
+
+// Octant slot assignment: slot bit a set <=> child lies on the high side of
+// axis a. child_in_slot[s]: the child in slot s, -1 for none.
+__device__ __forceinline__ void octant_slots(const float clo[8][3], const float chi[8][3], const float nlo[3], const float nhi[3], int nc,
+                                             int child_in_slot[8]) {
     int slot_of[8];
-    int child_in_slot[8];
     for (int s = 0; s < 8; s++) child_in_slot[s] = -1;
     for (int k = 0; k < 8; k++) slot_of[k] = -1;
     float ctr[3];
@@ -410,17 +381,11 @@ __global__ void k_collapse(const QItem *__restrict__ in, uint32_t n_in, QItem *_
         slot_of[bk] = bs;
         child_in_slot[bs] = bk;
     }
-    int n_internal = 0, n_leaf_tris = 0;
-    for (int k = 0; k < nc; k++) {
-        const uint32_t cnt = bin_count(c[k], first, last);
-        if (cnt > (uint32_t)LEAF_MAX_TRIS) n_internal++;
-        else n_leaf_tris += (int)cnt;
-    }
-    const uint32_t child_base = n_internal ? atomicAdd(&counters[0], (uint32_t)n_internal) : 0u;
-    const uint32_t tri_base = n_leaf_tris ? atomicAdd(&counters[1], (uint32_t)n_leaf_tris) : 0u;
-    WideNode nd;
-    // quantisation frame per axis (exact decode, one quantum of margin)
-    double qs[3], qp[3];
+}
+
+// Quantisation frame of a node per axis (exact decode, one quantum of
+// margin) into nd.p and nd.e; qs, qp: the quantum and the origin.
+__device__ __forceinline__ void quant_frame(const float nlo[3], const float nhi[3], WideNode &nd, double qs[3], double qp[3]) {
     for (int a = 0; a < 3; a++) {
         const float lo = nlo[a], hi = nhi[a];
         const float M = fmaxf(fabsf(lo), fabsf(hi));
@@ -442,6 +407,53 @@ __global__ void k_collapse(const QItem *__restrict__ in, uint32_t n_in, QItem *_
         nd.p[a] = (float)p;
         nd.e[a] = (uint8_t)(e + 127);
     }
+}
+
+// The box [lo, hi] in slot s of a node with frame (qs, qp): rounded outward
+// plus one quantum.
+__device__ __forceinline__ void quant_slot(const float lo[3], const float hi[3], int s, const double qs[3], const double qp[3], WideNode &nd) {
+    for (int a = 0; a < 3; a++) {
+        const int ql = (int)floor(__dsub_rd((double)lo[a], qp[a]) / qs[a]) - 1;
+        const int qh = (int)ceil(__dsub_ru((double)hi[a], qp[a]) / qs[a]) + 1;
+        nd.qlo[a][s] = (uint8_t)min(max(ql, 0), 255);
+        nd.qhi[a][s] = (uint8_t)min(max(qh, 0), 255);
+    }
+}
+
+__global__ void k_collapse(const QItem *__restrict__ in, uint32_t n_in, QItem *__restrict__ out, uint32_t *__restrict__ counters,
+                           const float *__restrict__ aabb, const uint32_t *__restrict__ sorted, const TriRec *__restrict__ tris_ref,
+                           const uint32_t *__restrict__ left, const uint32_t *__restrict__ right, const uint32_t *__restrict__ first,
+                           const uint32_t *__restrict__ last, const float *__restrict__ nb, const uint8_t *__restrict__ dec,
+                           const uint8_t *__restrict__ open_k, WideNode *__restrict__ nodes, TriRec *__restrict__ leaf_tris) {
+    // counters: [0] wide nodes allocated, [1] leaf triangles allocated,
+    //           [2] items written to `out`, [3] maximum depth
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n_in) return;
+    const QItem it = in[t];
+    uint32_t c[8];
+    const int nc = chosen_slots(it.bin, left, right, dec, open_k, c);
+    float clo[8][3], chi[8][3];
+    float nlo[3] = {INFINITY, INFINITY, INFINITY}, nhi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int k = 0; k < nc; k++) {
+        child_box(c[k], aabb, sorted, nb, clo[k], chi[k]);
+        for (int a = 0; a < 3; a++) {
+            nlo[a] = fminf(nlo[a], clo[k][a]);
+            nhi[a] = fmaxf(nhi[a], chi[k][a]);
+        }
+    }
+    int child_in_slot[8];
+    octant_slots(clo, chi, nlo, nhi, nc, child_in_slot);
+    int n_internal = 0, n_leaf_tris = 0;
+    for (int k = 0; k < nc; k++) {
+        const uint32_t cnt = bin_count(c[k], first, last);
+        if (cnt > (uint32_t)LEAF_MAX_TRIS) n_internal++;
+        else n_leaf_tris += (int)cnt;
+    }
+    const uint32_t child_base = n_internal ? atomicAdd(&counters[0], (uint32_t)n_internal) : 0u;
+    const uint32_t tri_base = n_leaf_tris ? atomicAdd(&counters[1], (uint32_t)n_leaf_tris) : 0u;
+    WideNode nd;
+    double qs[3], qp[3];
+    quant_frame(nlo, nhi, nd, qs, qp);
     nd.imask = 0;
     nd.child_base = child_base;
     nd.tri_base = tri_base;
@@ -453,12 +465,7 @@ __global__ void k_collapse(const QItem *__restrict__ in, uint32_t n_in, QItem *_
             for (int a = 0; a < 3; a++) { nd.qlo[a][s] = 0; nd.qhi[a][s] = 0; }
             continue;
         }
-        for (int a = 0; a < 3; a++) {
-            int ql = (int)floor(__dsub_rd((double)clo[k][a], qp[a]) / qs[a]) - 1;
-            int qh = (int)ceil(__dsub_ru((double)chi[k][a], qp[a]) / qs[a]) + 1;
-            nd.qlo[a][s] = (uint8_t)min(max(ql, 0), 255);
-            nd.qhi[a][s] = (uint8_t)min(max(qh, 0), 255);
-        }
+        quant_slot(clo[k], chi[k], s, qs, qp, nd);
         const uint32_t cnt = bin_count(c[k], first, last);
         if (cnt > (uint32_t)LEAF_MAX_TRIS) {
             nd.imask |= (uint8_t)(1u << s);
@@ -481,6 +488,106 @@ __global__ void k_collapse(const QItem *__restrict__ in, uint32_t n_in, QItem *_
     }
     nodes[it.wide] = nd;
     atomicMax(&counters[3], it.depth + 1);
+}
+
+// The instance tree's collapse, as k_collapse with one instance per leaf
+// slot: the topology only (imask, bases, meta and slot_src); k_tlas_boxes
+// fills in the boxes. counters as k_collapse's.
+__global__ void k_tlas_collapse(const QItem *__restrict__ in, uint32_t n_in, QItem *__restrict__ out, uint32_t *__restrict__ counters,
+                                const float *__restrict__ aabb, const uint32_t *__restrict__ sorted, const uint32_t *__restrict__ left,
+                                const uint32_t *__restrict__ right, const float *__restrict__ nb, const uint8_t *__restrict__ dec,
+                                const uint8_t *__restrict__ open_k, WideNode *__restrict__ nodes, uint32_t *__restrict__ slot_src,
+                                uint32_t *__restrict__ order) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n_in) return;
+    const QItem it = in[t];
+    uint32_t c[8];
+    const int nc = chosen_slots(it.bin, left, right, dec, open_k, c);
+    float clo[8][3], chi[8][3];
+    float nlo[3] = {INFINITY, INFINITY, INFINITY}, nhi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    int n_internal = 0;
+    for (int k = 0; k < nc; k++) {
+        child_box(c[k], aabb, sorted, nb, clo[k], chi[k]);
+        for (int a = 0; a < 3; a++) {
+            nlo[a] = fminf(nlo[a], clo[k][a]);
+            nhi[a] = fmaxf(nhi[a], chi[k][a]);
+        }
+        if (!(c[k] & LEAF)) n_internal++;
+    }
+    int child_in_slot[8];
+    octant_slots(clo, chi, nlo, nhi, nc, child_in_slot);
+    const uint32_t child_base = n_internal ? atomicAdd(&counters[0], (uint32_t)n_internal) : 0u;
+    const uint32_t inst_base = nc > n_internal ? atomicAdd(&counters[1], (uint32_t)(nc - n_internal)) : 0u;
+    WideNode nd{};
+    nd.child_base = child_base;
+    nd.tri_base = inst_base;
+    uint32_t rank = 0, off = 0;
+    for (int s = 0; s < 8; s++) {
+        const int k = child_in_slot[s];
+        uint32_t src = INST_EMPTY;
+        if (k >= 0 && !(c[k] & LEAF)) {
+            nd.imask |= (uint8_t)(1u << s);
+            nd.meta[s] = (uint8_t)((1u << 5) | (24u + (uint32_t)s));
+            src = child_base + rank;
+            out[atomicAdd(&counters[2], 1u)] = QItem{c[k], src, it.depth + 1};
+            rank++;
+        } else if (k >= 0) {
+            nd.meta[s] = (uint8_t)((1u << 5) | off);
+            const uint32_t m = sorted[c[k] & ~LEAF];
+            order[inst_base + off] = m;
+            src = INST_LEAF | m;
+            off++;
+        }
+        slot_src[8ull * it.wide + s] = src;
+    }
+    nodes[it.wide] = nd;
+}
+
+// Boxes of the instance tree's nodes [first, first + count), one level, the
+// deeper levels done: from the instances' world boxes and the child nodes'. A
+// node over a box that is not finite (an instance placed by a transform with
+// infinities or NaN) gets an infinite quantum, which leaves all its planes
+// unbounded in the traversal: its instances are left to their own test.
+__global__ void k_tlas_boxes(uint32_t first, uint32_t count, const float *__restrict__ aabb, const uint32_t *__restrict__ slot_src,
+                             float *__restrict__ box, WideNode *__restrict__ nodes) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= count) return;
+    const uint32_t i = first + t;
+    float nlo[3] = {INFINITY, INFINITY, INFINITY}, nhi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    bool finite = true;
+    for (int s = 0; s < 8; s++) {
+        const uint32_t src = slot_src[8ull * i + s];
+        if (src == INST_EMPTY) continue;
+        const float *b = (src & INST_LEAF) ? aabb + 6ull * (src & ~INST_LEAF) : box + 6ull * src;
+        for (int a = 0; a < 3; a++) {
+            finite = finite && isfinite(b[a]) && isfinite(b[3 + a]);
+            nlo[a] = fminf(nlo[a], b[a]);
+            nhi[a] = fmaxf(nhi[a], b[3 + a]);
+        }
+    }
+    WideNode nd = nodes[i];
+    if (finite) {
+        double qs[3], qp[3];
+        quant_frame(nlo, nhi, nd, qs, qp);
+        for (int s = 0; s < 8; s++) {
+            const uint32_t src = slot_src[8ull * i + s];
+            if (src == INST_EMPTY) continue;
+            const float *b = (src & INST_LEAF) ? aabb + 6ull * (src & ~INST_LEAF) : box + 6ull * src;
+            quant_slot(b, b + 3, s, qs, qp, nd);
+        }
+    } else {
+        for (int a = 0; a < 3; a++) {
+            nd.p[a] = 0.0f;
+            nd.e[a] = 255;
+            nlo[a] = -INFINITY;
+            nhi[a] = INFINITY;
+        }
+    }
+    nodes[i] = nd;
+    for (int a = 0; a < 3; a++) {
+        box[6ull * i + a] = nlo[a];
+        box[6ull * i + 3 + a] = nhi[a];
+    }
 }
 
 template <typename T>
@@ -564,7 +671,7 @@ int build_mesh_bvh(const TriRec *tris_ref, const float *aabb, uint32_t n, MeshBv
         k_bottom_up<<<(n + 255) / 256, 256, 0, st>>>(aabb, vals, (int)n, left, right, parent, nb, flags);
         RG_CUDA_TRY(cudaGetLastError());
         RG_CUDA_TRY(cudaMemsetAsync(flags, 0, ni * sizeof(uint32_t), st));
-        k_wide_cost<<<(n + 255) / 256, 256, 0, st>>>(aabb, vals, (int)n, left, right, parent, first, last, nb, flags, cost, dec, open_k);
+        k_wide_cost<LEAF_MAX_TRIS><<<(n + 255) / 256, 256, 0, st>>>(aabb, vals, (int)n, left, right, parent, first, last, nb, flags, cost, dec, open_k);
         RG_CUDA_TRY(cudaGetLastError());
         root_bin = 0;
     }
@@ -613,10 +720,72 @@ int build_mesh_bvh(const TriRec *tris_ref, const float *aabb, uint32_t n, MeshBv
 }
 
 void free_inst_tree(InstTree &t) {
-    void *ps[] = {t.aabb, t.sorted, t.left, t.right, t.parent, t.first, t.last, t.nb, t.flags, t.nodes};
+    void *ps[] = {t.aabb, t.order, t.nodes, t.slot_src, t.box};
     for (void *p : ps)
         if (p) cudaFree(p);
     t = InstTree{};
+}
+
+// The topology over n instance boxes (t.aabb).
+static int build_inst_topology(uint32_t n, InstTree &t, cudaStream_t st) {
+    const uint32_t ni = n - 1;
+    TmpAllocs tmp;
+    uint64_t *keys = nullptr;
+    uint32_t *sorted, *bounds, *left, *right, *parent, *first, *last, *flags, *counters;
+    float *nb, *cost;
+    uint8_t *dec, *open_k;
+    QItem *qa, *qb;
+    char *scratch = nullptr;
+    RG_CUDA_TRY(tmp.get(&keys, n));
+    RG_CUDA_TRY(tmp.get(&sorted, n));
+    RG_CUDA_TRY(tmp.get(&bounds, 6));
+    RG_CUDA_TRY(tmp.get(&left, ni));
+    RG_CUDA_TRY(tmp.get(&right, ni));
+    RG_CUDA_TRY(tmp.get(&parent, 2 * (size_t)n));
+    RG_CUDA_TRY(tmp.get(&first, ni));
+    RG_CUDA_TRY(tmp.get(&last, ni));
+    RG_CUDA_TRY(tmp.get(&flags, ni));
+    RG_CUDA_TRY(tmp.get(&counters, 4));
+    RG_CUDA_TRY(tmp.get(&nb, 6 * (size_t)ni));
+    RG_CUDA_TRY(tmp.get(&cost, 8 * (size_t)ni));
+    RG_CUDA_TRY(tmp.get(&dec, 8 * (size_t)ni));
+    RG_CUDA_TRY(tmp.get(&open_k, ni));
+    RG_CUDA_TRY(tmp.get(&qa, n));
+    RG_CUDA_TRY(tmp.get(&qb, n));
+    RG_CUDA_TRY(tmp.get(&scratch, radix_sort_scratch_bytes(n, 8)));
+    const uint32_t init_bounds[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
+    RG_CUDA_TRY(cudaMemcpyAsync(bounds, init_bounds, sizeof(init_bounds), cudaMemcpyHostToDevice, st));
+    k_bounds<<<std::min<uint32_t>((n + 255) / 256, 1184), 256, 0, st>>>(t.aabb, n, bounds);
+    k_morton<<<(n + 255) / 256, 256, 0, st>>>(t.aabb, n, bounds, keys, sorted);
+    RG_CUDA_TRY(cudaGetLastError());
+    RG_CUDA_TRY(radix_sort_pairs(keys, sorted, n, 8, 0, 64, scratch, st));
+    RG_CUDA_TRY(cudaMemsetAsync(flags, 0, ni * sizeof(uint32_t), st));
+    k_karras<<<(ni + 255) / 256, 256, 0, st>>>(keys, (int)n, left, right, parent, first, last);
+    k_bottom_up<<<(n + 255) / 256, 256, 0, st>>>(t.aabb, sorted, (int)n, left, right, parent, nb, flags);
+    RG_CUDA_TRY(cudaMemsetAsync(flags, 0, ni * sizeof(uint32_t), st));
+    k_wide_cost<1><<<(n + 255) / 256, 256, 0, st>>>(t.aabb, sorted, (int)n, left, right, parent, first, last, nb, flags, cost, dec, open_k);
+    RG_CUDA_TRY(cudaGetLastError());
+    const uint32_t init_counters[4] = {1u, 0u, 0u, 0u};
+    RG_CUDA_TRY(cudaMemcpyAsync(counters, init_counters, sizeof(init_counters), cudaMemcpyHostToDevice, st));
+    const QItem root{0u, 0u, 0u};
+    RG_CUDA_TRY(cudaMemcpyAsync(qa, &root, sizeof(root), cudaMemcpyHostToDevice, st));
+    t.level.assign(1, 0u);
+    for (uint32_t n_in = 1; n_in > 0;) {
+        t.level.push_back(t.level.back() + n_in);
+        if (t.level.back() > ni || t.level.size() > 200) {
+            set_error("instance tree collapse did not terminate");
+            return RAY_ERR_CUDA;
+        }
+        RG_CUDA_TRY(cudaMemsetAsync(counters + 2, 0, sizeof(uint32_t), st));
+        k_tlas_collapse<<<(n_in + 127) / 128, 128, 0, st>>>(qa, n_in, qb, counters, t.aabb, sorted, left, right, nb, dec, open_k, t.nodes,
+                                                           t.slot_src, t.order);
+        RG_CUDA_TRY(cudaGetLastError());
+        RG_CUDA_TRY(cudaMemcpyAsync(&n_in, counters + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        RG_CUDA_TRY(wait_stream(st)); // (also before the temporaries are freed)
+        std::swap(qa, qb);
+    }
+    t.count = t.level.back();
+    return RAY_OK;
 }
 
 int build_inst_tree(const float *boxes, uint32_t n, bool refit, InstTree &t, cudaStream_t st) {
@@ -624,44 +793,24 @@ int build_inst_tree(const float *boxes, uint32_t n, bool refit, InstTree &t, cud
         free_inst_tree(t);
         return RAY_OK;
     }
-    const uint32_t ni = n - 1;
     if (!refit || t.n != n) {
         free_inst_tree(t);
         RG_CUDA_TRY(dalloc(&t.aabb, 6 * (size_t)n));
-        RG_CUDA_TRY(dalloc(&t.sorted, n));
-        RG_CUDA_TRY(dalloc(&t.left, ni));
-        RG_CUDA_TRY(dalloc(&t.right, ni));
-        RG_CUDA_TRY(dalloc(&t.parent, 2 * (size_t)n));
-        RG_CUDA_TRY(dalloc(&t.first, ni));
-        RG_CUDA_TRY(dalloc(&t.last, ni));
-        RG_CUDA_TRY(dalloc(&t.nb, 6 * (size_t)ni));
-        RG_CUDA_TRY(dalloc(&t.flags, ni));
-        RG_CUDA_TRY(dalloc(&t.nodes, ni));
-        TmpAllocs tmp;
-        uint64_t *keys = nullptr;
-        uint32_t *bounds = nullptr;
-        char *scratch = nullptr;
-        RG_CUDA_TRY(tmp.get(&keys, n));
-        RG_CUDA_TRY(tmp.get(&bounds, 6));
-        RG_CUDA_TRY(tmp.get(&scratch, radix_sort_scratch_bytes(n, 8)));
+        RG_CUDA_TRY(dalloc(&t.order, n));
+        RG_CUDA_TRY(dalloc(&t.nodes, n - 1)); // at most one wide node per binary node
+        RG_CUDA_TRY(dalloc(&t.slot_src, 8 * (size_t)(n - 1)));
+        RG_CUDA_TRY(dalloc(&t.box, 6 * (size_t)(n - 1)));
         RG_CUDA_TRY(cudaMemcpyAsync(t.aabb, boxes, 6 * sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, st));
-        const uint32_t init_bounds[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-        RG_CUDA_TRY(cudaMemcpyAsync(bounds, init_bounds, sizeof(init_bounds), cudaMemcpyHostToDevice, st));
-        k_bounds<<<std::min<uint32_t>((n + 255) / 256, 1184), 256, 0, st>>>(t.aabb, n, bounds);
-        k_morton<<<(n + 255) / 256, 256, 0, st>>>(t.aabb, n, bounds, keys, t.sorted);
-        RG_CUDA_TRY(cudaGetLastError());
-        RG_CUDA_TRY(radix_sort_pairs(keys, t.sorted, n, 8, 0, 64, scratch, st));
-        k_karras<<<(ni + 255) / 256, 256, 0, st>>>(keys, (int)n, t.left, t.right, t.parent, t.first, t.last);
-        RG_CUDA_TRY(cudaGetLastError());
-        RG_CUDA_TRY(wait_stream(st)); // before the temporaries are freed
+        const int rc = build_inst_topology(n, t, st);
+        if (rc != RAY_OK) return rc;
         t.n = n;
     } else {
         RG_CUDA_TRY(cudaMemcpyAsync(t.aabb, boxes, 6 * sizeof(float) * (size_t)n, cudaMemcpyHostToDevice, st));
     }
-    // node boxes bottom-up (a refit: the same topology, the instances' new boxes), then the packed nodes
-    RG_CUDA_TRY(cudaMemsetAsync(t.flags, 0, ni * sizeof(uint32_t), st));
-    k_bottom_up<<<(n + 255) / 256, 256, 0, st>>>(t.aabb, t.sorted, (int)n, t.left, t.right, t.parent, t.nb, t.flags);
-    k_tlas_pack<<<(ni + 255) / 256, 256, 0, st>>>(t.aabb, t.sorted, (int)n, t.left, t.right, t.nb, t.nodes);
+    for (size_t l = t.level.size() - 1; l-- > 0;) {
+        const uint32_t first = t.level[l], count = t.level[l + 1] - first;
+        k_tlas_boxes<<<(count + 63) / 64, 64, 0, st>>>(first, count, t.aabb, t.slot_src, t.box, t.nodes);
+    }
     RG_CUDA_TRY(cudaGetLastError());
     return RAY_OK;
 }

@@ -577,7 +577,8 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     tp.refill_min = scn[0]->tuning.refill_min;
     for (int j = 0; j < n_jobs; j++) {
         bounces = std::max(bounces, jobs[j].bounces);
-        tp.max_depth = std::max(tp.max_depth, scn[j]->tuning.deep_stack ? 0xffffffffu : scn[j]->max_depth);
+        const uint32_t levels = scn[j]->max_depth + (scn[j]->tlas.nodes ? tlas_stack_levels(scn[j]->tlas.depth()) : 0u);
+        tp.max_depth = std::max(tp.max_depth, scn[j]->tuning.deep_stack ? 0xffffffffu : levels);
         if (scn[j]->tlas.nodes) tp.tlas = true; // the kernels that can walk an instance tree
     }
     tp.block = scn[0]->tuning.block;
@@ -690,7 +691,7 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     for (int q = 0; q < 2; q++) key.add(rays[q]).add(pay[q]).add(job[q]);
     key.add(hits).add(obj).add(cnt).add(shadow.recs).add(shadow.rays).add(shadow.job).add(rb->d_loop_sort.p).add(nee).add(ref_lights).add(principled_only);
     key.add(sv.nodes).add(sv.leaf_tris).add(sv.inst).add(sv.n_inst).add(tp.persistent).add(tp.refill_min).add(tp.max_depth).add(tp.views);
-    key.add(sv.tlas).add(tp.tlas).add(tp.block).add(tp.smem_stack).add(tp.one_tri);
+    key.add(sv.tlas).add(sv.tlas_inst).add(sv.tlas_count).add(tp.tlas).add(tp.block).add(tp.smem_stack).add(tp.one_tri);
     key.add(ev).add(geo_best).add(geo_tris).add(persp);
     return graph_run(*gs, key.h, st, enqueue);
 }

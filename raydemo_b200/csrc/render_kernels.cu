@@ -101,27 +101,15 @@ __device__ __forceinline__ void gen_primary(const CameraDev &cam, float k, float
     p.pad[0] = p.pad[1] = p.pad[2] = 0;
 }
 
-// Closest hit of one ray against the whole scene: the instance loop of
-// Traverse_MacroTree_WithStack_ClosestHit (CoreRef.cpp:1133-1222), as the
-// trace kernels run it.
+// Closest hit of one ray against the whole scene (Traverse_MacroTree_
+// WithStack_ClosestHit, CoreRef.cpp:1133-1222), as the trace kernels run it.
 __device__ __forceinline__ Best trace_closest_scene(const SceneView &sv, float4 r0, float4 r1, Stack<true> &st, uint32_t &err) {
     Best best;
     best.t = r0.w;
     best.u = best.v = 0.0f;
     best.prim = best.obj = -1;
-    const float sx = trav::safe_inv(r1.x), sy = trav::safe_inv(r1.y), sz = trav::safe_inv(r1.z);
     uint32_t nvis = 0, ntri = 0;
-    for (uint32_t m = 0; m < sv.n_inst; m++) {
-        const InstanceRec *ir = sv.inst + m;
-        float bmin[3], bmax[3];
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            bmin[q] = __ldg(&ir->bbox_min[q]);
-            bmax[q] = __ldg(&ir->bbox_max[q]);
-        }
-        if (!trav::ref_bbox_test(r0.x, r0.y, r0.z, sx, sy, sz, best.t, bmin, bmax)) continue;
-        trav::trace_mesh<false>(trav::mesh_of(sv, ir, (int)m), trav::transform_ray(ir, r0, r1), best, st, err, nvis, ntri);
-    }
+    trav::trace_scene<false, false>(sv, r0, r1, best, st, err, nvis, ntri);
     return best;
 }
 

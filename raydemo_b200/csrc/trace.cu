@@ -30,6 +30,10 @@ namespace {
 
 using namespace trav;
 
+// shared stack entries of the counting, any-hit and multi-scene launches
+constexpr int LOOP_STACK = 16;
+constexpr uint32_t MI_DONE = 0xfffffffeu; // no further instance of the ray to look for
+
 template <bool COUNT>
 __device__ __forceinline__ void flush_counters(uint32_t err, uint32_t nvis, uint32_t ntri, uint32_t *err_out, unsigned long long *counters) {
     if (err) atomicOr(err_out, err);
@@ -66,28 +70,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK) k_trace_closest(SceneView sv, con
         best.u = best.v = 0.0f;
         best.prim = -1;
         best.obj = -1;
-        const float sx = safe_inv(r1.x), sy = safe_inv(r1.y), sz = safe_inv(r1.z);
-        if (TLAS && sv.tlas) { // the instance tree
-            uint32_t tstk[TLAS_STACK];
-            int tsp = 1;
-            tstk[0] = 0;
-            for (int m; (m = tlas_next(sv, r0, sx, sy, sz, best.t, tstk, tsp, err)) >= 0;) {
-                const InstanceRec *ir = sv.inst + m;
-                trace_mesh<COUNT>(mesh_of(sv, ir, m), transform_ray(ir, r0, r1), best, st, err, nvis, ntri);
-            }
-        } else {
-            for (uint32_t m = 0; m < sv.n_inst; m++) {
-                const InstanceRec *ir = sv.inst + m;
-                float bmin[3], bmax[3];
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    bmin[k] = __ldg(&ir->bbox_min[k]);
-                    bmax[k] = __ldg(&ir->bbox_max[k]);
-                }
-                if (!ref_bbox_test(r0.x, r0.y, r0.z, sx, sy, sz, best.t, bmin, bmax)) continue;
-                trace_mesh<COUNT>(mesh_of(sv, ir, (int)m), transform_ray(ir, r0, r1), best, st, err, nvis, ntri);
-            }
-        }
+        trace_scene<COUNT, TLAS>(sv, r0, r1, best, st, err, nvis, ntri);
         hits[i] = make_float4(__int_as_float(best.prim), best.t, best.prim >= 0 ? best.u : 0.0f, best.prim >= 0 ? best.v : 0.0f);
         if (obj_out) obj_out[i] = best.obj;
     }
@@ -121,19 +104,34 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
     st.sp = 0;
     uint32_t err = 0, nvis = 0, ntri = 0;
     uint32_t ri = NO_RAY, mi = 0, visits = 0;
-    uint32_t tstk[TLAS ? TLAS_STACK : 1]; // the ray's instance-tree stack (scenes with an instance tree)
-    int tsp = 0;
-    bool in_mesh = false;
+    bool in_mesh = false; // traversing a mesh, or the instance tree (in_tree)
+    bool in_tree = false;
+    int sp0 = 0; // stack entries below the mesh's own (the tree's groups)
     constexpr bool BEST_SMEM = (SDEPTH * 8 + 12) * BLOCK <= 48 * 1024;
     __shared__ float s_best[BEST_SMEM ? 3 * BLOCK : 1];
     LaneBest<BLOCK, BEST_SMEM> best;
     best.t = 0.0f;
     best.prim = -1;
     if constexpr (BEST_SMEM) best.slot = s_best + threadIdx.x;
+    // the ray in world space (origin, reciprocals) and the tree's visit count,
+    // kept while the lane is inside an instance
+    constexpr bool WORLD_SMEM = TLAS && (SDEPTH * 8 + 12 + 28) * BLOCK <= 48 * 1024;
+    __shared__ float s_world[WORLD_SMEM ? 7 * BLOCK : 1];
+    float *const world = s_world + (WORLD_SMEM ? threadIdx.x : 0);
     LocalRay r = make_local_ray(0.0f, 0.0f, 0.0f, 1.0f, 1.0f, 1.0f);
     MeshRef mr{};
     uint32_t ng_base = 0, ng_bits = 0, tg_base = 0, tg_bits = 0;
     bool pool_empty = false;
+    auto scene_of = [&](uint32_t ray) -> const SceneView & {
+        return *reinterpret_cast<const SceneView *>(views + (size_t)__ldg(ray_job + ray) * view_stride);
+    };
+    auto enter = [&](const SceneView &lsv, const InstanceRec *ir, int m, float4 r0, float4 r1) {
+        mr = mesh_of(lsv, ir, m);
+        r = transform_ray(ir, r0, r1);
+        ng_base = 0;
+        ng_bits = r.root_bits();
+        visits = 0;
+    };
     while (true) {
         // ---- refill lanes that have no ray
         const uint32_t need = __ballot_sync(0xffffffffu, ri == NO_RAY);
@@ -148,10 +146,6 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
                 if (idx < n) {
                     ri = order ? __ldg(order + idx) : idx;
                     mi = 0;
-                    if (TLAS) {
-                        tstk[0] = 0; // the tree's root, for a scene that has one
-                        tsp = 1;
-                    }
                     in_mesh = false;
                     best.t = __ldg(&rays[2ull * ri].w);
                     best.prim = -1;
@@ -165,61 +159,61 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
         // (one triangle per step, 4M-ray launch of the microbench on B200:
         // 4.28 ms without, 3.7 ms with)
         bool idle = ri == NO_RAY;
-        // ---- next instance whose box the ray enters, or the end of the ray
-        // (a ray whose scene has no instance left is done without reading it
-        // again; a multi-scene ray reads its scene view first)
+        // ---- the start of the ray (its scene's instance tree, or the first
+        // instance whose box it enters), the next instance, or the end of the
+        // ray (a ray whose scene has no instance left is done without reading
+        // it again; a multi-scene ray reads its scene view first)
         if (!idle && !in_mesh) {
-          if (MULTI || (TLAS && sv.tlas ? tsp > 0 : mi < sv.n_inst)) {
-            // streaming hint: the ray is read once per instance pass and the
-            // hit written once, so they may leave L1/L2 first (evict-first),
-            // which keeps more of the BVH resident
-            const float4 r0 = stream_hint ? __ldcs(rays + 2ull * ri) : __ldg(rays + 2ull * ri);
-            const float4 r1 = stream_hint ? __ldcs(rays + 2ull * ri + 1) : __ldg(rays + 2ull * ri + 1);
-            const float sx = safe_inv(r1.x), sy = safe_inv(r1.y), sz = safe_inv(r1.z);
-            SceneView job_sv;
-            if (MULTI) job_sv = *reinterpret_cast<const SceneView *>(views + (size_t)__ldg(ray_job + ri) * view_stride);
-            const SceneView &lsv = MULTI ? job_sv : sv;
-            if (TLAS && lsv.tlas) {
-                const int m = tlas_next(lsv, r0, sx, sy, sz, best.t, tstk, tsp, err);
-                if (m >= 0) {
-                    const InstanceRec *ir = lsv.inst + m;
-                    mr = mesh_of(lsv, ir, m);
-                    r = transform_ray(ir, r0, r1);
+            if (mi < MI_DONE && (MULTI || mi < sv.n_inst)) {
+                // streaming hint: the ray is read once per instance pass and the
+                // hit written once, so they may leave L1/L2 first (evict-first),
+                // which keeps more of the BVH resident
+                const float4 r0 = stream_hint ? __ldcs(rays + 2ull * ri) : __ldg(rays + 2ull * ri);
+                const float4 r1 = stream_hint ? __ldcs(rays + 2ull * ri + 1) : __ldg(rays + 2ull * ri + 1);
+                const float sx = safe_inv(r1.x), sy = safe_inv(r1.y), sz = safe_inv(r1.z);
+                const SceneView &lsv = MULTI ? scene_of(ri) : sv;
+                st.sp = 0;
+                sp0 = 0;
+                tg_bits = 0;
+                if (TLAS && lsv.tlas) {
+                    mi = MI_DONE; // no instance after the tree's
+                    r = world_ray(r0.x, r0.y, r0.z, sx, sy, sz);
+                    if (WORLD_SMEM) {
+                        world[0] = r.ox;
+                        world[BLOCK] = r.oy;
+                        world[2 * BLOCK] = r.oz;
+                        world[3 * BLOCK] = r.ix;
+                        world[4 * BLOCK] = r.iy;
+                        world[5 * BLOCK] = r.iz;
+                    }
+                    mr = tree_of(lsv);
                     ng_base = 0;
                     ng_bits = r.root_bits();
-                    tg_bits = 0;
-                    st.sp = 0;
                     visits = 0;
-                    in_mesh = true;
+                    in_mesh = in_tree = true;
                 }
-            }
-            while ((!TLAS || !lsv.tlas) && mi < lsv.n_inst) {
-                const InstanceRec *ir = lsv.inst + mi;
-                float bmin[3], bmax[3];
+                while ((!TLAS || !lsv.tlas) && mi < lsv.n_inst) {
+                    const InstanceRec *ir = lsv.inst + mi;
+                    float bmin[3], bmax[3];
 #pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    bmin[k] = __ldg(&ir->bbox_min[k]);
-                    bmax[k] = __ldg(&ir->bbox_max[k]);
+                    for (int k = 0; k < 3; k++) {
+                        bmin[k] = __ldg(&ir->bbox_min[k]);
+                        bmax[k] = __ldg(&ir->bbox_max[k]);
+                    }
+                    mi++;
+                    if (!ref_bbox_test(r0.x, r0.y, r0.z, sx, sy, sz, best.t, bmin, bmax)) continue;
+                    enter(lsv, ir, (int)mi - 1, r0, r1);
+                    in_mesh = true;
+                    if (TLAS) in_tree = false;
+                    break;
                 }
-                mi++;
-                if (!ref_bbox_test(r0.x, r0.y, r0.z, sx, sy, sz, best.t, bmin, bmax)) continue;
-                mr = mesh_of(lsv, ir, (int)mi - 1);
-                r = transform_ray(ir, r0, r1);
-                ng_base = 0;
-                ng_bits = r.root_bits();
-                tg_bits = 0;
-                st.sp = 0;
-                visits = 0;
-                in_mesh = true;
-                break;
             }
-          }
             if (!in_mesh) {
                 const bool found = best.prim >= 0;
                 const float4 h = make_float4(__int_as_float(best.prim), best.t, found ? best.u() : 0.0f, found ? best.v() : 0.0f);
                 if (stream_hint) __stcs(hits + ri, h);
                 else hits[ri] = h;
-                if (obj_out) obj_out[ri] = found ? best.obj() : -1;
+                if (obj_out) obj_out[ri] = found ? best.obj_of() : -1;
                 ri = NO_RAY;
                 idle = true;
             }
@@ -230,17 +224,42 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
         if (!idle && tg_bits == 0) {
             if (!node_step<COUNT>(mr, r, best.t, ng_base, ng_bits, tg_base, tg_bits, st, visits, err, nvis)) {
                 in_mesh = false;
-                mi = 0xffffffffu; // abandon the ray; the error flag reports it
-                tsp = 0;
+                mi = MI_DONE; // abandon the ray; the error flag reports it
                 tg_bits = 0;
                 idle = true;
             }
         }
         __syncwarp();
+        // ---- instances: a lane whose tree node has leaf entries left takes the
+        // next one the ray enters; the rest of the node waits on the stack
+        if (TLAS) {
+            if (!idle && in_tree && tg_bits) {
+                const SceneView &lsv = MULTI ? scene_of(ri) : sv;
+                const int m = next_instance(lsv, r, best.t, tg_base, tg_bits, err);
+                if (m >= 0) {
+                    bool ok = ng_bits <= 0x00FFFFFFu || st.push(make_uint2(ng_base, ng_bits));
+                    if (tg_bits) ok = st.push(make_uint2(tg_base, tg_bits)) && ok;
+                    tg_bits = 0;
+                    if (ok) {
+                        const float4 r0 = __ldg(rays + 2ull * ri), r1 = __ldg(rays + 2ull * ri + 1);
+                        if (WORLD_SMEM) world[6 * BLOCK] = __uint_as_float(visits);
+                        enter(lsv, lsv.inst + m, m, r0, r1);
+                        in_tree = false;
+                        sp0 = st.sp;
+                    } else {
+                        err |= TRACE_ERR_STACK;
+                        in_mesh = false;
+                        mi = MI_DONE;
+                        idle = true;
+                    }
+                }
+            }
+            __syncwarp();
+        }
         // ---- triangles: one per lane, then (not with ONE) the others
         bool stop = false;
         while (true) {
-            if (!idle && tg_bits) {
+            if (!idle && tg_bits && !(TLAS && in_tree)) {
                 const uint32_t k = __ffs(tg_bits) - 1;
                 tg_bits &= tg_bits - 1;
                 if (ANY) {
@@ -252,23 +271,40 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
                     tri_test<COUNT>(mr, r, tg_base + k, best, err, ntri);
                 }
             }
-            if (ONE || !__any_sync(0xffffffffu, !idle && tg_bits)) break;
+            if (ONE || !__any_sync(0xffffffffu, !idle && tg_bits && !(TLAS && in_tree))) break;
         }
         __syncwarp();
         if (idle) continue;
         if (ANY && stop) { // a solid triangle blocks the ray: no further instance
             in_mesh = false;
-            mi = 0xffffffffu;
-            tsp = 0;
+            mi = MI_DONE;
             continue;
         }
         if (tg_bits == 0 && ng_bits <= 0x00FFFFFFu) {
-            if (st.sp == 0) {
+            if (TLAS && !in_tree && mi == MI_DONE && st.sp == sp0) { // the instance is done: back to the tree
+                if (WORLD_SMEM) {
+                    r = world_ray(world[0], world[BLOCK], world[2 * BLOCK], world[3 * BLOCK], world[4 * BLOCK], world[5 * BLOCK]);
+                    visits = __float_as_uint(world[6 * BLOCK]);
+                } else {
+                    const float4 r0 = __ldg(rays + 2ull * ri), r1 = __ldg(rays + 2ull * ri + 1);
+                    r = world_ray(r0.x, r0.y, r0.z, safe_inv(r1.x), safe_inv(r1.y), safe_inv(r1.z));
+                    visits = 0;
+                }
+                mr = tree_of(MULTI ? scene_of(ri) : sv);
+                in_tree = true;
+                sp0 = 0;
+            }
+            if (st.sp == sp0) {
                 in_mesh = false;
             } else {
                 const uint2 e = st.pop();
-                ng_base = e.x;
-                ng_bits = e.y;
+                if (!TLAS || e.y > 0x00FFFFFFu) {
+                    ng_base = e.x;
+                    ng_bits = e.y;
+                } else { // the rest of a tree node's leaf entries
+                    tg_base = e.x;
+                    tg_bits = e.y;
+                }
             }
         }
     }
@@ -361,7 +397,7 @@ cudaError_t launch_tuned_dispatch(const SceneView &sv, const float4 *rays, uint3
 template <bool DEEP, bool TLAS>
 cudaError_t launch_impl(const SceneView &sv, const float4 *rays, uint32_t n, float4 *hits, int32_t *obj, uint32_t *err,
                         unsigned long long *counters, bool count, cudaStream_t st, const TraceParams &tp) {
-    constexpr int B = TRACE_BLOCK, D = SMEM_STACK;
+    constexpr int B = TRACE_BLOCK, D = LOOP_STACK;
     if (!tp.persistent && !tp.views && !tp.any) {
         const uint32_t grid = (n + TRACE_BLOCK - 1) / TRACE_BLOCK;
         if (count)
@@ -371,7 +407,7 @@ cudaError_t launch_impl(const SceneView &sv, const float4 *rays, uint32_t n, flo
         return cudaGetLastError();
     }
     if (!tp.next_ray) return cudaErrorInvalidValue;
-    if (!count && !tp.views && !tp.any && (tp.one_tri || !(tp.block == TRACE_BLOCK && tp.smem_stack == SMEM_STACK)))
+    if (!count && !tp.views && !tp.any)
         return launch_tuned_dispatch<DEEP, TLAS>(sv, rays, n, hits, obj, err, counters, st, tp);
     int &blocks = g_persistent_blocks[DEEP ? 1 : 0][TLAS ? 1 : 0];
     if (blocks == 0) {
@@ -406,12 +442,8 @@ cudaError_t launch_impl(const SceneView &sv, const float4 *rays, uint32_t n, flo
         return cudaGetLastError();
     }
 #undef RG_LAUNCH_P
-    if (count)
-        k_trace_persistent<true, DEEP, false, false, B, D, TLAS><<<blocks, TRACE_BLOCK, 0, st>>>(
-            sv, rays, n, hits, obj, err, counters, tp.next_ray, tp.refill_min, tp.count, nullptr, 0, nullptr, tp.order);
-    else
-        k_trace_persistent<false, DEEP, false, false, B, D, TLAS><<<blocks, TRACE_BLOCK, 0, st>>>(
-            sv, rays, n, hits, obj, err, counters, tp.next_ray, tp.refill_min, tp.count, nullptr, 0, nullptr, tp.order, tp.stream_hint);
+    k_trace_persistent<true, DEEP, false, false, B, D, TLAS><<<blocks, TRACE_BLOCK, 0, st>>>(
+        sv, rays, n, hits, obj, err, counters, tp.next_ray, tp.refill_min, tp.count, nullptr, 0, nullptr, tp.order);
     return cudaGetLastError();
 }
 
@@ -421,9 +453,9 @@ cudaError_t launch_trace_closest(const SceneView &sv, const float4 *rays, uint32
                                  unsigned long long *counters, bool count, cudaStream_t st, const TraceParams &tp) {
     if (n == 0) return cudaSuccess;
     // one group per level at most: the shared-memory stack suffices up to its
-    // depth in levels (the tuned closest-hit kernel's depth where it applies)
-    const bool tuned = tp.persistent && !count && !tp.views && !tp.any;
-    const uint32_t sdepth = tuned ? (uint32_t)tp.smem_stack : (uint32_t)SMEM_STACK;
+    // depth in levels
+    const bool special = count || tp.views || tp.any;
+    const uint32_t sdepth = tp.persistent || tp.views || tp.any ? (special ? (uint32_t)LOOP_STACK : (uint32_t)tp.smem_stack) : (uint32_t)SMEM_STACK;
     if (tp.tlas) {
         if (tp.max_depth < sdepth) return launch_impl<false, true>(sv, rays, n, hits, obj, err, counters, count, st, tp);
         return launch_impl<true, true>(sv, rays, n, hits, obj, err, counters, count, st, tp);

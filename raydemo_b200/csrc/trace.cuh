@@ -11,21 +11,30 @@ struct SceneView {
     const TriRec *leaf_tris;
     const InstanceRec *inst;
     uint32_t n_inst;
-    // the instance tree (n_inst - 1 nodes), or null: the traversal then tests
+    // the instance tree (tlas_count wide nodes over the instances' world boxes;
+    // leaf entry k is instance tlas_inst[k]), or null: the traversal then tests
     // the instances' boxes one after another
-    const TlasNode *tlas = nullptr;
+    const WideNode *tlas = nullptr;
+    const uint32_t *tlas_inst = nullptr;
+    uint32_t tlas_count = 0;
 };
 
 // Instance counts from which traces walk the instance tree instead of
-// testing every instance box in turn.
-constexpr uint32_t TLAS_MIN_INSTANCES = 32;
+// testing every instance box in turn: one wide node holds 8 boxes. Measured
+// on B200 (1M incoherent rays, spheres of 1,280 triangles, in turn / tree):
+// 4 instances 271 / 290 us, 8 314 / 307, 16 442 / 342, 64 1348 / 507.
+constexpr uint32_t TLAS_MIN_INSTANCES = 8;
+// Stack entries a ray holds at most beside its mesh's while it traverses an
+// instance of a tree of the given depth: a group per tree level, and the
+// rest of the leaf group it came from.
+constexpr uint32_t tlas_stack_levels(uint32_t tlas_depth) { return tlas_depth + 1; }
 
 // Error bits written (OR-ed) to *err by the traversal.
 constexpr uint32_t TRACE_ERR_STACK = 1u;
 constexpr uint32_t TRACE_ERR_BOUNDS = 2u; // a node or triangle index outside the mesh's arrays
 constexpr uint32_t TRACE_ERR_LIMIT = 4u;  // more node visits than the mesh has nodes
 // (8 is the radix sort's look-back bound, SORT_ERR_LOOKBACK)
-constexpr uint32_t TRACE_ERR_TLAS = 16u;  // the instance tree's stack overflowed or an index was out of bounds
+constexpr uint32_t TRACE_ERR_TLAS = 16u;  // an instance index of the tree out of bounds
 
 // Kernel choice and its knobs (picked by the tuner).
 struct TraceParams {
@@ -42,7 +51,9 @@ struct TraceParams {
     // closest-hit persistent kernel: rays read and hits written with the
     // streaming (evict-first) cache hint
     int stream_hint = 0;
-    uint32_t max_depth = 0; // deepest wide BVH among the traced meshes (sizes the stack)
+    // deepest wide BVH among the traced meshes, plus what an instance tree adds
+    // (tlas_stack_levels): sizes the stack
+    uint32_t max_depth = 0;
     uint32_t *next_ray = nullptr; // device work counter for the persistent kernel
     const uint32_t *count = nullptr; // device ray count: when set, min(n, *count) rays are traced
     // rays of several scenes (persistent kernel only): ray i is traced in the
@@ -51,7 +62,7 @@ struct TraceParams {
     uint32_t view_stride = 0;
     const uint32_t *ray_job = nullptr;
     // some scene of the launch has an instance tree: the kernels that walk it
-    // (the others test the instance boxes in turn and carry no tree stack)
+    // (the others test the instance boxes in turn)
     bool tlas = false;
     // trace order: the k-th ray taken is ray order[k] (its hit is written at
     // that index); null: input order

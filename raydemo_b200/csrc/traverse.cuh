@@ -71,27 +71,6 @@ __device__ __forceinline__ bool ref_bbox_test(float ox, float oy, float oz, floa
     return tmin <= tmax && tmin <= t && tmax > 0;
 }
 
-// The same slab test, also giving the entry distance (for visiting order).
-// For a box containing another, it accepts whenever the test on the inner
-// box accepts (every rounding step is monotonic), so an instance-tree node
-// is never culled where the reference's test enters one of its instances.
-__device__ __forceinline__ bool ref_bbox_entry(float ox, float oy, float oz, float ix, float iy, float iz, float t, const float *bmin,
-                                               const float *bmax, float &tmin_out) {
-    float lo_x = __fmul_rn(ix, __fsub_rn(bmin[0], ox)), hi_x = __fmul_rn(ix, __fsub_rn(bmax[0], ox));
-    if (lo_x > hi_x) { const float tmp = lo_x; lo_x = hi_x; hi_x = tmp; }
-    float lo_y = __fmul_rn(iy, __fsub_rn(bmin[1], oy)), hi_y = __fmul_rn(iy, __fsub_rn(bmax[1], oy));
-    if (lo_y > hi_y) { const float tmp = lo_y; lo_y = hi_y; hi_y = tmp; }
-    float lo_z = __fmul_rn(iz, __fsub_rn(bmin[2], oz)), hi_z = __fmul_rn(iz, __fsub_rn(bmax[2], oz));
-    if (lo_z > hi_z) { const float tmp = lo_z; lo_z = hi_z; hi_z = tmp; }
-    float tmin = lo_x > lo_y ? lo_x : lo_y;
-    if (lo_z > tmin) tmin = lo_z;
-    float tmax = hi_x < hi_y ? hi_x : hi_y;
-    if (hi_z < tmax) tmax = hi_z;
-    tmax = __fmul_rn(tmax, 1.00000024f);
-    tmin_out = tmin;
-    return tmin <= tmax && tmin <= t && tmax > 0;
-}
-
 // safe_invert, CoreRef.cpp:272-294
 __device__ __forceinline__ float safe_inv(float v) {
     float r = __frcp_rn(v);
@@ -108,6 +87,7 @@ struct Best {
         v = v_;
         obj = obj_;
     }
+    __device__ __forceinline__ int obj_of() const { return obj; }
 };
 
 // The best hit of a lane of the persistent kernel: what the tests compare
@@ -133,7 +113,7 @@ struct LaneBest<STRIDE, false> {
     }
     __device__ __forceinline__ float u() const { return bu; }
     __device__ __forceinline__ float v() const { return bv; }
-    __device__ __forceinline__ int obj() const { return bobj; }
+    __device__ __forceinline__ int obj_of() const { return bobj; }
 };
 
 template <int STRIDE>
@@ -148,7 +128,7 @@ struct LaneBest<STRIDE, true> {
     }
     __device__ __forceinline__ float u() const { return slot[0]; }
     __device__ __forceinline__ float v() const { return slot[STRIDE]; }
-    __device__ __forceinline__ int obj() const { return __float_as_int(slot[2 * STRIDE]); }
+    __device__ __forceinline__ int obj_of() const { return __float_as_int(slot[2 * STRIDE]); }
 };
 
 // Ray in the space of the instance being traversed.
@@ -246,57 +226,57 @@ __device__ __forceinline__ MeshRef mesh_of(const SceneView &sv, const InstanceRe
     return mr;
 }
 
-// Instance-tree walk, one ray: pops entries of the ray's instance stack
-// (stk, sp) until an instance whose world box the ray enters with the
-// current best t -- the reference's instance test, bbox_test with the
-// safe-inverted direction -- and returns its index; -1 when the walk is
-// done. An internal node pushes the children whose boxes the ray enters,
-// the nearer on top; an instance pushed this way is tested again when popped
-// (best t may have shrunk). Indices outside the tree and a full stack set
-// TRACE_ERR_TLAS (the walk goes on without the entry).
-constexpr int TLAS_STACK = 48;
-__device__ __forceinline__ int tlas_next(const SceneView &sv, float4 r0, float sx, float sy, float sz, float best_t, uint32_t *stk, int &sp,
-                                         uint32_t &err) {
-    while (sp > 0) {
-        const uint32_t e = stk[--sp];
-        if (e & TLAS_LEAF) {
-            const uint32_t m = e & ~TLAS_LEAF;
-            if (m >= sv.n_inst) {
-                err |= TRACE_ERR_TLAS;
-                continue;
-            }
-            const InstanceRec *ir = sv.inst + m;
-            float bmin[3], bmax[3];
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                bmin[k] = __ldg(&ir->bbox_min[k]);
-                bmax[k] = __ldg(&ir->bbox_max[k]);
-            }
-            if (ref_bbox_test(r0.x, r0.y, r0.z, sx, sy, sz, best_t, bmin, bmax)) return (int)m;
-            continue;
-        }
-        if (e + 1 >= sv.n_inst) {
+// The ray in world space, as the instance tree is traversed: the reciprocals
+// are the instance test's own (safe_invert), so a component of 1e-7 or less
+// counts as zero there and here. With all three that small nothing is left to
+// order the axes by: the planes alone decide (they come out unbounded where
+// they overflow).
+__device__ __forceinline__ LocalRay world_ray(float ox, float oy, float oz, float ix, float iy, float iz) {
+    LocalRay r;
+    r.ox = ox; r.oy = oy; r.oz = oz;
+    r.dx = r.dy = r.dz = 0.0f;
+    r.ix = ix; r.iy = iy; r.iz = iz;
+    r.oct = (ix < 0.0f ? 1u : 0u) | (iy < 0.0f ? 2u : 0u) | (iz < 0.0f ? 4u : 0u);
+    const float big = 3.402823466e+38F;
+    const uint32_t zero = (fabsf(ix) == big ? 8u : 0u) | (fabsf(iy) == big ? 16u : 0u) | (fabsf(iz) == big ? 32u : 0u);
+    if (zero != 56u) r.oct |= zero;
+    return r;
+}
+
+// The instance tree as the node step takes it. A leaf entry's test is the
+// reference's own instance test (bbox_test with safe_invert), so no instance
+// is entered that the reference culls; the nodes above accept whatever that
+// test accepts. With the test's reciprocals, its near plane errs by 2u of its
+// t and its far plane, widened by 1 + 4u, by 7u; the node step's slack of 16u
+// (|B| + 33024|A|), 3u of which its own rounding takes, covers both, and the
+// node's planes lie a quantum outside the instance's box besides.
+__device__ __forceinline__ MeshRef tree_of(const SceneView &sv) {
+    MeshRef mr;
+    mr.nodes = sv.tlas;
+    mr.tris = nullptr;
+    mr.prim_base = 0;
+    mr.node_count = sv.tlas_count;
+    mr.tri_count = sv.n_inst;
+    mr.obj = -1;
+    return mr;
+}
+
+// The next instance of a leaf group of the tree (tg_base, tg_bits) that the
+// ray enters with the current best t, taken out of the group; -1 for none.
+__device__ __forceinline__ int next_instance(const SceneView &sv, const LocalRay &w, float best_t, uint32_t tg_base, uint32_t &tg_bits,
+                                             uint32_t &err) {
+    while (tg_bits) {
+        const uint32_t e = tg_base + __ffs(tg_bits) - 1u;
+        tg_bits &= tg_bits - 1u;
+        const uint32_t m = e < sv.n_inst ? __ldg(sv.tlas_inst + e) : 0xffffffffu;
+        if (m >= sv.n_inst) {
             err |= TRACE_ERR_TLAS;
             continue;
         }
-        const float4 *np = reinterpret_cast<const float4 *>(sv.tlas + e);
-        const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
-        const uint4 ids = __ldg(reinterpret_cast<const uint4 *>(np + 3));
-        const float lo0[3] = {a.x, a.y, a.z}, lo1[3] = {a.w, b.x, b.y}, hi0[3] = {b.z, b.w, c.x}, hi1[3] = {c.y, c.z, c.w};
-        float t0 = 0.0f, t1 = 0.0f;
-        const bool h0 = ref_bbox_entry(r0.x, r0.y, r0.z, sx, sy, sz, best_t, lo0, hi0, t0);
-        const bool h1 = ref_bbox_entry(r0.x, r0.y, r0.z, sx, sy, sz, best_t, lo1, hi1, t1);
-        const bool near1 = h1 && (!h0 || t1 < t0); // child 1 first when it is the nearer (or the only) one
-        const uint32_t first = near1 ? ids.y : ids.x, second = near1 ? ids.x : ids.y;
-        const bool has_second = h0 && h1;
-        if (has_second) {
-            if (sp < TLAS_STACK) stk[sp++] = second;
-            else err |= TRACE_ERR_TLAS;
-        }
-        if (h0 || h1) {
-            if (sp < TLAS_STACK) stk[sp++] = first;
-            else err |= TRACE_ERR_TLAS;
-        }
+        const InstanceRec *ir = sv.inst + m;
+        const float4 lo = __ldg(reinterpret_cast<const float4 *>(ir->bbox_min)), hi = __ldg(reinterpret_cast<const float4 *>(ir->bbox_max));
+        const float bmin[3] = {lo.x, lo.y, lo.z}, bmax[3] = {hi.x, hi.y, hi.z};
+        if (ref_bbox_test(w.ox, w.oy, w.oz, w.ix, w.iy, w.iz, best_t, bmin, bmax)) return (int)m;
     }
     return -1;
 }
@@ -360,11 +340,12 @@ __device__ __forceinline__ bool node_step(const MeshRef &mr, const LocalRay &r, 
     // It is evaluated as one FMA on the byte read as the float v = 2^15 + q:
     // t = v * A + (B - 2^15 A), v * A exact inside the FMA. Rounding
     // B - 2^15 A, then -/+ slack, then the FMA's result errs by less than
-    // 3u(|B| + 33024|A|) (u = 2^-24); the slack 2^-21 (|B| + 33024|A|)
+    // 3u(|B| + 33024|A|) (u = 2^-24); the slack 2^-20 (|B| + 33024|A|)
     // moves the near planes down and the far planes up by more than that,
     // so the test accepts every box that the exact slab test on the decoded
-    // box accepts. (An overflowing 2^15 A gives NaN planes: that axis is
-    // left unbounded, still conservative.)
+    // box accepts, and with the instance tree what the instance test accepts
+    // (tree_of). (An overflowing 2^15 A gives NaN planes: that axis is left
+    // unbounded, still conservative.)
     // The step is bound by instruction issue. The set-up of the x and y axes
     // goes through packed arithmetic; the children's FMAs stay scalar, packed
     // ones measured slower (the pairs' registers spill at 64 a thread: 3.41
@@ -382,7 +363,7 @@ __device__ __forceinline__ bool node_step(const MeshRef &mr, const LocalRay &r, 
     const float Sz = __fmaf_rn(fabsf(Az), 33024.0f, fabsf(Bz));
     const unsigned long long B0xy = fma2(Axy, pack2(-32768.0f, -32768.0f), Bxy);
     const float B0z = __fmaf_rn(-32768.0f, Az, Bz);
-    constexpr float SLACK = 4.76837158203125e-07f; // 2^-21
+    constexpr float SLACK = 9.5367431640625e-07f; // 2^-20
     const unsigned long long Bnxy = fma2(Sxy, pack2(-SLACK, -SLACK), B0xy), Bfxy = fma2(Sxy, pack2(SLACK, SLACK), B0xy);
     const float Bnz = __fmaf_rn(Sz, -SLACK, B0z), Bfz = __fmaf_rn(Sz, SLACK, B0z);
     float Bnx, Bny, Bfx, Bfy;
@@ -472,7 +453,9 @@ __device__ __forceinline__ bool tri_test(const MeshRef &mr, const LocalRay &r, u
     if (tri_core(t0, t1, t2, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, rdet, dett, detu, detv)) {
         const float t = __fmul_rn(dett, rdet);
         const int gp = (int)(mr.prim_base + __float_as_uint(t2.z));
-        if (t > 0.0f && (t < best.t || (t == best.t && best.prim >= 0 && gp < best.prim))) {
+        // a tie goes to the lower triangle index, then to the lower instance:
+        // independent of the visiting order
+        if (t > 0.0f && (t < best.t || (t == best.t && best.prim >= 0 && gp <= best.prim && (gp < best.prim || mr.obj < best.obj_of())))) {
             best.t = t;
             best.prim = gp;
             best.rest(__fmul_rn(detu, rdet), __fmul_rn(detv, rdet), mr.obj);
@@ -490,7 +473,7 @@ __device__ __forceinline__ void trace_mesh(const MeshRef &mr, const LocalRay &r,
                                            uint32_t &nvis, uint32_t &ntri) {
     uint32_t ng_base = 0, ng_bits = r.root_bits();
     uint32_t tg_base = 0, tg_bits = 0, visits = 0;
-    st.sp = 0;
+    const int sp0 = st.sp; // the caller's entries below
     while (true) {
         if (!node_step<COUNT>(mr, r, best.t, ng_base, ng_bits, tg_base, tg_bits, st, visits, err, nvis)) return;
         while (tg_bits) {
@@ -499,7 +482,7 @@ __device__ __forceinline__ void trace_mesh(const MeshRef &mr, const LocalRay &r,
             tri_test<COUNT>(mr, r, tg_base + k, best, err, ntri);
         }
         if (ng_bits <= 0x00FFFFFFu) {
-            if (st.sp == 0) return;
+            if (st.sp == sp0) return;
             const uint2 e = st.pop();
             ng_base = e.x;
             ng_bits = e.y;
@@ -528,6 +511,48 @@ __device__ __forceinline__ bool trace_mesh_any(const MeshRef &mr, const LocalRay
             ng_base = e.x;
             ng_bits = e.y;
         }
+    }
+}
+
+// Closest hit of one ray (r0, r1) against the whole scene, one thread: the
+// instances of the tree where the scene has one, else all in turn.
+template <bool COUNT, bool TLAS, typename ST>
+__device__ __forceinline__ void trace_scene(const SceneView &sv, float4 r0, float4 r1, Best &best, ST &st, uint32_t &err, uint32_t &nvis,
+                                            uint32_t &ntri) {
+    const float sx = safe_inv(r1.x), sy = safe_inv(r1.y), sz = safe_inv(r1.z);
+    if (TLAS && sv.tlas) {
+        const MeshRef tree = tree_of(sv);
+        const LocalRay w = world_ray(r0.x, r0.y, r0.z, sx, sy, sz);
+        uint32_t ng_base = 0, ng_bits = w.root_bits(), tg_base = 0, tg_bits = 0, visits = 0, none = 0;
+        st.sp = 0;
+        while (true) {
+            if (ng_bits > 0x00FFFFFFu && !node_step<false>(tree, w, best.t, ng_base, ng_bits, tg_base, tg_bits, st, visits, err, none)) return;
+            const int floor_sp = st.sp;
+            for (int m; (m = next_instance(sv, w, best.t, tg_base, tg_bits, err)) >= 0;) {
+                // the mesh's groups go on top of the tree's
+                const InstanceRec *ir = sv.inst + m;
+                trace_mesh<COUNT>(mesh_of(sv, ir, m), transform_ray(ir, r0, r1), best, st, err, nvis, ntri);
+                st.sp = floor_sp;
+            }
+            if (ng_bits <= 0x00FFFFFFu) {
+                if (st.sp == 0) return;
+                const uint2 e = st.pop();
+                ng_base = e.x;
+                ng_bits = e.y;
+            }
+        }
+    }
+    for (uint32_t m = 0; m < sv.n_inst; m++) {
+        const InstanceRec *ir = sv.inst + m;
+        float bmin[3], bmax[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            bmin[k] = __ldg(&ir->bbox_min[k]);
+            bmax[k] = __ldg(&ir->bbox_max[k]);
+        }
+        if (!ref_bbox_test(r0.x, r0.y, r0.z, sx, sy, sz, best.t, bmin, bmax)) continue;
+        st.sp = 0;
+        trace_mesh<COUNT>(mesh_of(sv, ir, (int)m), transform_ray(ir, r0, r1), best, st, err, nvis, ntri);
     }
 }
 
