@@ -19,9 +19,17 @@
 //                        incoherent rays of very different lengths
 //   k_trace_closest_one  its closest-hit, one-triangle-per-step form for
 //                        scenes without an instance tree, register-bounded
+// The persistent kernels trace a ray with eight lanes, one per child of a
+// node and one per triangle of a leaf, where rays are few: launches of at most
+// one wave of such groups, and every launch's last rays (a warp with no more
+// than four left and none to take). There a ray's steps follow one another
+// with nothing to hide them, and a step's latency is what counts.
 // The stack holds one node group per tree level at most. It lives in shared
 // memory; meshes deeper than that use the DEEP instances, which continue it
 // in a local array.
+#include <algorithm>
+#include <type_traits>
+
 #include "trace.cuh"
 #include "traverse.cuh"
 
@@ -33,6 +41,13 @@ using namespace trav;
 // shared stack entries of the counting, any-hit and multi-scene launches
 constexpr int LOOP_STACK = 16;
 constexpr uint32_t MI_DONE = 0xfffffffeu; // no further instance of the ray to look for
+
+// Ray counts up to which a launch traces every ray with eight lanes: as many
+// groups of eight as the resident grid has. Measured on B200 (20,000
+// triangles, one lane / eight lanes a ray): 100 rays 77 / 57 us, 1,000 109 /
+// 75, 10,000 111 / 100, 20,000 116 / 113; beyond one wave of groups the single
+// lanes win (40,000 rays 134 / 162).
+constexpr uint32_t coop_rays(int blocks, int block) { return (uint32_t)blocks * (uint32_t)block / 8u; }
 
 template <bool COUNT>
 __device__ __forceinline__ void flush_counters(uint32_t err, uint32_t nvis, uint32_t ntri, uint32_t *err_out, unsigned long long *counters) {
@@ -96,7 +111,8 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
                                                  int32_t *__restrict__ obj_out, uint32_t *__restrict__ err_out,
                                                  unsigned long long *__restrict__ counters, uint32_t *__restrict__ next_ray, int refill_min,
                                                  const uint32_t *__restrict__ n_dev, const uint8_t *__restrict__ views, uint32_t view_stride,
-                                                 const uint32_t *__restrict__ ray_job, const uint32_t *__restrict__ order, int stream_hint) {
+                                                 const uint32_t *__restrict__ ray_job, const uint32_t *__restrict__ order, int stream_hint,
+                                                 uint32_t coop_max) {
     if (n_dev) n = min(n, *n_dev);
     __shared__ uint2 s_stack[SDEPTH * BLOCK];
     Stack<DEEP, BLOCK, SDEPTH> st;
@@ -117,7 +133,7 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
     // kept while the lane is inside an instance
     constexpr bool WORLD_SMEM = TLAS && (SDEPTH * 8 + 12 + 28) * BLOCK <= 48 * 1024;
     __shared__ float s_world[WORLD_SMEM ? 7 * BLOCK : 1];
-    float *const world = s_world + (WORLD_SMEM ? threadIdx.x : 0);
+    float *world = s_world + (WORLD_SMEM ? threadIdx.x : 0);
     LocalRay r = make_local_ray(0.0f, 0.0f, 0.0f, 1.0f, 1.0f, 1.0f);
     MeshRef mr{};
     uint32_t ng_base = 0, ng_bits = 0, tg_base = 0, tg_bits = 0;
@@ -132,7 +148,114 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
         ng_bits = r.root_bits();
         visits = 0;
     };
-    while (true) {
+    // The start of a lane's ray (its scene's instance tree, or the first
+    // instance whose box it enters) or its next instance; false when the ray
+    // is done (a ray whose scene has no instance left is done without reading
+    // it again; a multi-scene ray reads its scene view first).
+    auto next_mesh = [&]() -> bool {
+        if (mi >= MI_DONE || !(MULTI || mi < sv.n_inst)) return false;
+        // streaming hint: the ray is read once per instance pass and the
+        // hit written once, so they may leave L1/L2 first (evict-first),
+        // which keeps more of the BVH resident
+        const float4 r0 = stream_hint ? __ldcs(rays + 2ull * ri) : __ldg(rays + 2ull * ri);
+        const float4 r1 = stream_hint ? __ldcs(rays + 2ull * ri + 1) : __ldg(rays + 2ull * ri + 1);
+        const float sx = safe_inv(r1.x), sy = safe_inv(r1.y), sz = safe_inv(r1.z);
+        const SceneView &lsv = MULTI ? scene_of(ri) : sv;
+        st.sp = 0;
+        sp0 = 0;
+        tg_bits = 0;
+        if (TLAS && lsv.tlas) {
+            mi = MI_DONE; // no instance after the tree's
+            r = world_ray(r0.x, r0.y, r0.z, sx, sy, sz);
+            if (WORLD_SMEM) { // (a group's eight lanes write the same values)
+                world[0] = r.ox;
+                world[BLOCK] = r.oy;
+                world[2 * BLOCK] = r.oz;
+                world[3 * BLOCK] = r.ix;
+                world[4 * BLOCK] = r.iy;
+                world[5 * BLOCK] = r.iz;
+            }
+            mr = tree_of(lsv);
+            ng_base = 0;
+            ng_bits = r.root_bits();
+            visits = 0;
+            in_tree = true;
+            return true;
+        }
+        while (mi < lsv.n_inst) {
+            const InstanceRec *ir = lsv.inst + mi;
+            float bmin[3], bmax[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                bmin[k] = __ldg(&ir->bbox_min[k]);
+                bmax[k] = __ldg(&ir->bbox_max[k]);
+            }
+            mi++;
+            if (!ref_bbox_test(r0.x, r0.y, r0.z, sx, sy, sz, best.t, bmin, bmax)) continue;
+            enter(lsv, ir, (int)mi - 1, r0, r1);
+            if (TLAS) in_tree = false;
+            return true;
+        }
+        return false;
+    };
+    auto write_hit = [&]() {
+        const bool found = best.prim >= 0;
+        const float4 h = make_float4(__int_as_float(best.prim), best.t, found ? best.u() : 0.0f, found ? best.v() : 0.0f);
+        if (stream_hint) __stcs(hits + ri, h);
+        else hits[ri] = h;
+        if (obj_out) obj_out[ri] = found ? best.obj_of() : -1;
+    };
+    // A lane whose tree node has leaf entries left takes the next instance the
+    // ray enters; the rest of the node waits on the stack. False: the stack is full.
+    auto enter_instance = [&](bool writer) -> bool {
+        const SceneView &lsv = MULTI ? scene_of(ri) : sv;
+        const int m = next_instance(lsv, r, best.t, tg_base, tg_bits, err);
+        if (m < 0) return true;
+        bool ok = ng_bits <= 0x00FFFFFFu || st.push_group(make_uint2(ng_base, ng_bits), writer);
+        if (tg_bits) ok = st.push_group(make_uint2(tg_base, tg_bits), writer) && ok;
+        tg_bits = 0;
+        if (!ok) {
+            err |= TRACE_ERR_STACK;
+            return false;
+        }
+        const float4 r0 = __ldg(rays + 2ull * ri), r1 = __ldg(rays + 2ull * ri + 1);
+        if (WORLD_SMEM) world[6 * BLOCK] = __uint_as_float(visits);
+        enter(lsv, lsv.inst + m, m, r0, r1);
+        in_tree = false;
+        sp0 = st.sp;
+        return true;
+    };
+    // The end of a group: the next one from the stack, the tree when an
+    // instance of it is done; false when the mesh (or the tree) is.
+    auto next_group = [&]() -> bool {
+        if (TLAS && !in_tree && mi == MI_DONE && st.sp == sp0) { // the instance is done: back to the tree
+            if (WORLD_SMEM) {
+                r = world_ray(world[0], world[BLOCK], world[2 * BLOCK], world[3 * BLOCK], world[4 * BLOCK], world[5 * BLOCK]);
+                visits = __float_as_uint(world[6 * BLOCK]);
+            } else {
+                const float4 r0 = __ldg(rays + 2ull * ri), r1 = __ldg(rays + 2ull * ri + 1);
+                r = world_ray(r0.x, r0.y, r0.z, safe_inv(r1.x), safe_inv(r1.y), safe_inv(r1.z));
+                visits = 0;
+            }
+            mr = tree_of(MULTI ? scene_of(ri) : sv);
+            in_tree = true;
+            sp0 = 0;
+        }
+        if (st.sp == sp0) return false;
+        const uint2 e = st.pop();
+        if (!TLAS || e.y > 0x00FFFFFFu) {
+            ng_base = e.x;
+            ng_bits = e.y;
+        } else { // the rest of a tree node's leaf entries
+            tg_base = e.x;
+            tg_bits = e.y;
+        }
+        return true;
+    };
+    // few rays: eight lanes each from the start
+    constexpr bool COOP = !COUNT;
+    const bool few = COOP && n <= coop_max;
+    while (!few) {
         // ---- refill lanes that have no ray
         const uint32_t need = __ballot_sync(0xffffffffu, ri == NO_RAY);
         if (!pool_empty && need != 0 && (__popc(need) >= refill_min || need == 0xffffffffu)) {
@@ -152,68 +275,22 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
                 }
             }
         }
-        if (pool_empty && __all_sync(0xffffffffu, ri == NO_RAY)) break;
+        if (pool_empty) {
+            // the launch's last rays: once a warp has no more than four left, eight lanes each
+            const uint32_t live = __ballot_sync(0xffffffffu, ri != NO_RAY);
+            if (live == 0 || (COOP && !DEEP && __popc(live) <= 4)) break;
+        }
         // A lane without work this iteration falls through to the next one, the
         // warp meeting again (__syncwarp) after each phase, which keeps lanes
         // that took different branches from drifting into different iterations
         // (one triangle per step, 4M-ray launch of the microbench on B200:
         // 4.28 ms without, 3.7 ms with)
         bool idle = ri == NO_RAY;
-        // ---- the start of the ray (its scene's instance tree, or the first
-        // instance whose box it enters), the next instance, or the end of the
-        // ray (a ray whose scene has no instance left is done without reading
-        // it again; a multi-scene ray reads its scene view first)
+        // ---- the start of the ray, the next instance, or the end of the ray
         if (!idle && !in_mesh) {
-            if (mi < MI_DONE && (MULTI || mi < sv.n_inst)) {
-                // streaming hint: the ray is read once per instance pass and the
-                // hit written once, so they may leave L1/L2 first (evict-first),
-                // which keeps more of the BVH resident
-                const float4 r0 = stream_hint ? __ldcs(rays + 2ull * ri) : __ldg(rays + 2ull * ri);
-                const float4 r1 = stream_hint ? __ldcs(rays + 2ull * ri + 1) : __ldg(rays + 2ull * ri + 1);
-                const float sx = safe_inv(r1.x), sy = safe_inv(r1.y), sz = safe_inv(r1.z);
-                const SceneView &lsv = MULTI ? scene_of(ri) : sv;
-                st.sp = 0;
-                sp0 = 0;
-                tg_bits = 0;
-                if (TLAS && lsv.tlas) {
-                    mi = MI_DONE; // no instance after the tree's
-                    r = world_ray(r0.x, r0.y, r0.z, sx, sy, sz);
-                    if (WORLD_SMEM) {
-                        world[0] = r.ox;
-                        world[BLOCK] = r.oy;
-                        world[2 * BLOCK] = r.oz;
-                        world[3 * BLOCK] = r.ix;
-                        world[4 * BLOCK] = r.iy;
-                        world[5 * BLOCK] = r.iz;
-                    }
-                    mr = tree_of(lsv);
-                    ng_base = 0;
-                    ng_bits = r.root_bits();
-                    visits = 0;
-                    in_mesh = in_tree = true;
-                }
-                while ((!TLAS || !lsv.tlas) && mi < lsv.n_inst) {
-                    const InstanceRec *ir = lsv.inst + mi;
-                    float bmin[3], bmax[3];
-#pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        bmin[k] = __ldg(&ir->bbox_min[k]);
-                        bmax[k] = __ldg(&ir->bbox_max[k]);
-                    }
-                    mi++;
-                    if (!ref_bbox_test(r0.x, r0.y, r0.z, sx, sy, sz, best.t, bmin, bmax)) continue;
-                    enter(lsv, ir, (int)mi - 1, r0, r1);
-                    in_mesh = true;
-                    if (TLAS) in_tree = false;
-                    break;
-                }
-            }
+            in_mesh = next_mesh();
             if (!in_mesh) {
-                const bool found = best.prim >= 0;
-                const float4 h = make_float4(__int_as_float(best.prim), best.t, found ? best.u() : 0.0f, found ? best.v() : 0.0f);
-                if (stream_hint) __stcs(hits + ri, h);
-                else hits[ri] = h;
-                if (obj_out) obj_out[ri] = found ? best.obj_of() : -1;
+                write_hit();
                 ri = NO_RAY;
                 idle = true;
             }
@@ -230,29 +307,12 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
             }
         }
         __syncwarp();
-        // ---- instances: a lane whose tree node has leaf entries left takes the
-        // next one the ray enters; the rest of the node waits on the stack
+        // ---- instances
         if (TLAS) {
-            if (!idle && in_tree && tg_bits) {
-                const SceneView &lsv = MULTI ? scene_of(ri) : sv;
-                const int m = next_instance(lsv, r, best.t, tg_base, tg_bits, err);
-                if (m >= 0) {
-                    bool ok = ng_bits <= 0x00FFFFFFu || st.push(make_uint2(ng_base, ng_bits));
-                    if (tg_bits) ok = st.push(make_uint2(tg_base, tg_bits)) && ok;
-                    tg_bits = 0;
-                    if (ok) {
-                        const float4 r0 = __ldg(rays + 2ull * ri), r1 = __ldg(rays + 2ull * ri + 1);
-                        if (WORLD_SMEM) world[6 * BLOCK] = __uint_as_float(visits);
-                        enter(lsv, lsv.inst + m, m, r0, r1);
-                        in_tree = false;
-                        sp0 = st.sp;
-                    } else {
-                        err |= TRACE_ERR_STACK;
-                        in_mesh = false;
-                        mi = MI_DONE;
-                        idle = true;
-                    }
-                }
+            if (!idle && in_tree && tg_bits && !enter_instance(true)) {
+                in_mesh = false;
+                mi = MI_DONE;
+                idle = true;
             }
             __syncwarp();
         }
@@ -280,32 +340,173 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
             mi = MI_DONE;
             continue;
         }
-        if (tg_bits == 0 && ng_bits <= 0x00FFFFFFu) {
-            if (TLAS && !in_tree && mi == MI_DONE && st.sp == sp0) { // the instance is done: back to the tree
-                if (WORLD_SMEM) {
-                    r = world_ray(world[0], world[BLOCK], world[2 * BLOCK], world[3 * BLOCK], world[4 * BLOCK], world[5 * BLOCK]);
-                    visits = __float_as_uint(world[6 * BLOCK]);
-                } else {
-                    const float4 r0 = __ldg(rays + 2ull * ri), r1 = __ldg(rays + 2ull * ri + 1);
-                    r = world_ray(r0.x, r0.y, r0.z, safe_inv(r1.x), safe_inv(r1.y), safe_inv(r1.z));
-                    visits = 0;
-                }
-                mr = tree_of(MULTI ? scene_of(ri) : sv);
-                in_tree = true;
-                sp0 = 0;
+        if (tg_bits == 0 && ng_bits <= 0x00FFFFFFu) in_mesh = next_group();
+    }
+    if constexpr (COOP) {
+        // ---- eight lanes per ray: the group's lanes hold the same state, the
+        // ray's stack, best hit and world ray being its owner's (a lane of the
+        // main loop whose ray it is, or the group's first lane)
+        const uint32_t lane = threadIdx.x & 31u, grp = lane >> 3, c = lane & 7u;
+        uint32_t live = few ? 0u : __ballot_sync(0xffffffffu, ri != NO_RAY);
+        if (!few && live == 0) {
+            flush_counters<COUNT>(err, nvis, ntri, err_out, counters);
+            return;
+        }
+        for (uint32_t k = 0; k < grp; k++) live &= live - 1u;
+        const bool has = live != 0;
+        const uint32_t own = has ? __ffs(live) - 1u : grp * 8u;
+        if (!few) { // hand over the ray's state
+            auto take = [&](auto &x) { x = __shfl_sync(0xffffffffu, x, own); };
+            auto take_flag = [&](bool &x) { x = __shfl_sync(0xffffffffu, (int)x, own) != 0; };
+            auto take_ptr = [&](auto *&x) {
+                x = reinterpret_cast<std::remove_reference_t<decltype(x)>>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(x), own));
+            };
+            take(ri);
+            take(mi);
+            take(visits);
+            take(sp0);
+            take(st.sp);
+            take_flag(in_mesh);
+            take_flag(in_tree);
+            take(best.t);
+            take(best.prim);
+            if constexpr (!BEST_SMEM) {
+                take(best.bu);
+                take(best.bv);
+                take(best.bobj);
             }
-            if (st.sp == sp0) {
+            take(r.ox);
+            take(r.oy);
+            take(r.oz);
+            take(r.dx);
+            take(r.dy);
+            take(r.dz);
+            take(r.ix);
+            take(r.iy);
+            take(r.iz);
+            take(r.oct);
+            take_ptr(mr.nodes);
+            take_ptr(mr.tris);
+            take(mr.prim_base);
+            take(mr.node_count);
+            take(mr.tri_count);
+            take(mr.obj);
+            take(ng_base);
+            take(ng_bits);
+            take(tg_base);
+            take(tg_bits);
+            if (!has) ri = NO_RAY;
+        }
+        const int off = (int)own - (int)lane;
+        st.smem += off;
+        if constexpr (BEST_SMEM) best.slot += off;
+        if (WORLD_SMEM) world += off;
+        __syncwarp();
+        // the groups that take rays: with fewer rays than warps one a warp (its
+        // steps then wait for no other ray's), else all four
+        const uint32_t takers = n <= gridDim.x * (BLOCK / 32) ? 1u : 0x01010101u;
+        while (true) {
+            if (few && !pool_empty) {
+                const uint32_t need = __ballot_sync(0xffffffffu, ri == NO_RAY) & takers; // the groups' first lanes
+                if (need) {
+                    uint32_t base = 0;
+                    const uint32_t leader = __ffs(need) - 1;
+                    if (lane == leader) base = atomicAdd(next_ray, (uint32_t)__popc(need));
+                    base = __shfl_sync(0xffffffffu, base, leader);
+                    if (base + __popc(need) >= n) pool_empty = true;
+                    if ((need >> (grp * 8u)) & 1u) {
+                        const uint32_t idx = base + __popc(need & ((1u << (grp * 8u)) - 1u));
+                        if (idx < n) {
+                            ri = order ? __ldg(order + idx) : idx;
+                            mi = 0;
+                            in_mesh = false;
+                            best.t = __ldg(&rays[2ull * ri].w);
+                            best.prim = -1;
+                        }
+                    }
+                }
+            }
+            if ((!few || pool_empty) && __all_sync(0xffffffffu, ri == NO_RAY)) break;
+            bool idle = ri == NO_RAY;
+            if (!idle && !in_mesh) {
+                in_mesh = next_mesh();
+                if (!in_mesh) {
+                    if (c == 0) write_hit();
+                    ri = NO_RAY;
+                    idle = true;
+                }
+            }
+            __syncwarp();
+            if (!node_step_coop(!idle && tg_bits == 0, mr, r, best.t, ng_base, ng_bits, tg_base, tg_bits, st, visits, err)) {
                 in_mesh = false;
-            } else {
-                const uint2 e = st.pop();
-                if (!TLAS || e.y > 0x00FFFFFFu) {
-                    ng_base = e.x;
-                    ng_bits = e.y;
-                } else { // the rest of a tree node's leaf entries
-                    tg_base = e.x;
-                    tg_bits = e.y;
+                mi = MI_DONE;
+                tg_bits = 0;
+                idle = true;
+            }
+            if (TLAS) {
+                if (!idle && in_tree && tg_bits && !enter_instance(c == 0)) {
+                    in_mesh = false;
+                    mi = MI_DONE;
+                    idle = true;
                 }
             }
+            // triangles: lane c the c-th of the group's list, eight at a time
+            bool stop = false;
+            const bool tri = !idle && !(TLAS && in_tree);
+            while (__any_sync(0xffffffffu, tri && tg_bits)) {
+                uint32_t m = tri ? tg_bits : 0u;
+                for (uint32_t k = 0; k < c; k++) m &= m - 1u;
+                float t = 0.0f, u = 0.0f, v = 0.0f;
+                int gp = 0;
+                bool solid = false;
+                const bool cand = m != 0 && tri_candidate(mr, r, tg_base + __ffs(m) - 1u, best, err, t, u, v, gp, solid);
+                if (tri) { // past the eight
+                    for (int k = 0; k < 8; k++) tg_bits &= tg_bits - 1u;
+                }
+                if (__any_sync(0xffffffffu, cand)) {
+                    // the group's winner: any hit prefers a solid triangle (it ends the ray); then the
+                    // nearest, a tie to the lower triangle
+                    uint32_t from = lane;
+                    uint32_t rank = !cand ? 2u : (ANY && solid ? 0u : 1u);
+                    float wt = t;
+                    int wp = gp;
+                    for (uint32_t o = 4; o; o >>= 1) {
+                        const uint32_t orank = __shfl_xor_sync(0xffffffffu, rank, o), ofrom = __shfl_xor_sync(0xffffffffu, from, o);
+                        const float ot = __shfl_xor_sync(0xffffffffu, wt, o);
+                        const int op = __shfl_xor_sync(0xffffffffu, wp, o);
+                        if (orank < rank || (orank == rank && (ot < wt || (ot == wt && op < wp)))) {
+                            rank = orank;
+                            from = ofrom;
+                            wt = ot;
+                            wp = op;
+                        }
+                    }
+                    if (rank < 2u) {
+                        best.t = wt;
+                        best.prim = wp;
+                        if (ANY && rank == 0u) {
+                            stop = true;
+                            tg_bits = 0;
+                        }
+                    }
+                    if constexpr (BEST_SMEM) {
+                        if (rank < 2u && from == lane) best.rest(u, v, mr.obj);
+                    } else {
+                        u = __shfl_sync(0xffffffffu, u, from);
+                        v = __shfl_sync(0xffffffffu, v, from);
+                        if (rank < 2u) best.rest(u, v, mr.obj);
+                    }
+                    __syncwarp();
+                }
+            }
+            __syncwarp(); // the groups' pushes before their pops
+            if (idle) continue;
+            if (ANY && stop) {
+                in_mesh = false;
+                mi = MI_DONE;
+                continue;
+            }
+            if (tg_bits == 0 && ng_bits <= 0x00FFFFFFu) in_mesh = next_group();
         }
     }
     flush_counters<COUNT>(err, nvis, ntri, err_out, counters);
@@ -319,9 +520,10 @@ __global__ void __launch_bounds__(BLOCK) k_trace_persistent(SceneView sv, const 
                                                                   uint32_t *__restrict__ next_ray, int refill_min,
                                                                   const uint32_t *__restrict__ n_dev, const uint8_t *__restrict__ views = nullptr,
                                                                   uint32_t view_stride = 0, const uint32_t *__restrict__ ray_job = nullptr,
-                                                                  const uint32_t *__restrict__ order = nullptr, int stream_hint = 0) {
+                                                                  const uint32_t *__restrict__ order = nullptr, int stream_hint = 0,
+                                                                  uint32_t coop_max = 0) {
     trace_persistent<COUNT, DEEP, MULTI, ANY, BLOCK, SDEPTH, TLAS, ONE>(sv, rays, n, hits, obj_out, err_out, counters, next_ray, refill_min,
-                                                                        n_dev, views, view_stride, ray_job, order, stream_hint);
+                                                                        n_dev, views, view_stride, ray_job, order, stream_hint, coop_max);
 }
 
 // The closest-hit, one-triangle-per-step form for scenes without an
@@ -337,9 +539,10 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_trace_closest_one(Scene
                                                                           unsigned long long *__restrict__ counters,
                                                                           uint32_t *__restrict__ next_ray, int refill_min,
                                                                           const uint32_t *__restrict__ n_dev,
-                                                                          const uint32_t *__restrict__ order, int stream_hint) {
+                                                                          const uint32_t *__restrict__ order, int stream_hint,
+                                                                          uint32_t coop_max) {
     trace_persistent<false, false, false, false, BLOCK, SDEPTH, false, true>(sv, rays, n, hits, obj_out, err_out, counters, next_ray,
-                                                                              refill_min, n_dev, nullptr, 0, nullptr, order, stream_hint);
+                                                                              refill_min, n_dev, nullptr, 0, nullptr, order, stream_hint, coop_max);
 }
 
 int g_persistent_blocks[2][2] = {{0, 0}, {0, 0}}; // [DEEP][TLAS]
@@ -371,12 +574,15 @@ cudaError_t launch_tuned(const SceneView &sv, const float4 *rays, uint32_t n, fl
     }
     cudaError_t e = cudaMemsetAsync(tp.next_ray, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
+    const uint32_t coop = coop_rays(blocks, BLOCK);
+    // few rays, the count known here: no more blocks than give each a warp
+    const uint32_t grid = n <= coop ? std::min<uint32_t>(blocks, (n + BLOCK / 32 - 1) / (BLOCK / 32)) : (uint32_t)blocks;
     if (FAST)
-        k_trace_closest_one<BLOCK, SDEPTH><<<blocks, BLOCK, 0, st>>>(sv, rays, n, hits, obj, err, counters, tp.next_ray, tp.refill_min, tp.count,
-                                                                     tp.order, tp.stream_hint);
+        k_trace_closest_one<BLOCK, SDEPTH><<<grid, BLOCK, 0, st>>>(sv, rays, n, hits, obj, err, counters, tp.next_ray, tp.refill_min, tp.count,
+                                                                     tp.order, tp.stream_hint, coop);
     else
-        k_trace_persistent<false, DEEP, false, false, BLOCK, SDEPTH, TLAS, ONE><<<blocks, BLOCK, 0, st>>>(
-            sv, rays, n, hits, obj, err, counters, tp.next_ray, tp.refill_min, tp.count, nullptr, 0, nullptr, tp.order, tp.stream_hint);
+        k_trace_persistent<false, DEEP, false, false, BLOCK, SDEPTH, TLAS, ONE><<<grid, BLOCK, 0, st>>>(
+            sv, rays, n, hits, obj, err, counters, tp.next_ray, tp.refill_min, tp.count, nullptr, 0, nullptr, tp.order, tp.stream_hint, coop);
     return cudaGetLastError();
 }
 
@@ -421,11 +627,12 @@ cudaError_t launch_impl(const SceneView &sv, const float4 *rays, uint32_t n, flo
     }
     cudaError_t e = cudaMemsetAsync(tp.next_ray, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
+    const uint32_t coop = coop_rays(blocks, TRACE_BLOCK);
     // shadow rays and rays of several scenes (no counting variants), with one
     // triangle test per step or a node's triangles at once
 #define RG_LAUNCH_P(MULTI_, ANY_, ONE_)                                                                                                 \
     k_trace_persistent<false, DEEP, MULTI_, ANY_, B, D, TLAS, ONE_><<<blocks, TRACE_BLOCK, 0, st>>>(                                    \
-        sv, rays, n, hits, obj, err, counters, tp.next_ray, tp.refill_min, tp.count, tp.views, tp.view_stride, tp.ray_job)
+        sv, rays, n, hits, obj, err, counters, tp.next_ray, tp.refill_min, tp.count, tp.views, tp.view_stride, tp.ray_job, nullptr, 0, coop)
     if (tp.any) {
         if (tp.views) {
             if (tp.one_tri) RG_LAUNCH_P(true, true, true);

@@ -12,6 +12,7 @@ constexpr int TRACE_BLOCK = 128;
 constexpr int SMEM_STACK = 24; // entries per thread in shared memory
 constexpr int LMEM_STACK = 40; // further entries in a local array (DEEP instances only)
 constexpr uint32_t NO_RAY = 0xffffffffu;
+constexpr float SLAB_SLACK = 9.5367431640625e-07f; // 2^-20, see node_step
 
 // Three-input max / min (sm_100). NaN inputs are dropped, as fmaxf/fminf drop them.
 __device__ __forceinline__ float max3f(float a, float b, float c) {
@@ -168,6 +169,13 @@ struct Stack<false, STRIDE, DEPTH> {
         sp--;
         return smem[sp * STRIDE];
     }
+    // eight lanes with one stack (the same smem): one of them writes
+    __device__ __forceinline__ bool push_group(uint2 e, bool writer) {
+        if (sp >= DEPTH) return false;
+        if (writer) smem[sp * STRIDE] = e;
+        sp++;
+        return true;
+    }
 };
 
 template <int STRIDE, int DEPTH>
@@ -186,6 +194,14 @@ struct Stack<true, STRIDE, DEPTH> {
     __device__ __forceinline__ uint2 pop() {
         sp--;
         return sp < DEPTH ? smem[sp * STRIDE] : lmem[sp - DEPTH];
+    }
+    // eight lanes with one stack: one writes the shared part, each its own copy of the rest
+    __device__ __forceinline__ bool push_group(uint2 e, bool writer) {
+        if (sp >= DEPTH + LOCAL) return false;
+        if (sp >= DEPTH) lmem[sp - DEPTH] = e;
+        else if (writer) smem[sp * STRIDE] = e;
+        sp++;
+        return true;
     }
 };
 
@@ -363,7 +379,7 @@ __device__ __forceinline__ bool node_step(const MeshRef &mr, const LocalRay &r, 
     const float Sz = __fmaf_rn(fabsf(Az), 33024.0f, fabsf(Bz));
     const unsigned long long B0xy = fma2(Axy, pack2(-32768.0f, -32768.0f), Bxy);
     const float B0z = __fmaf_rn(-32768.0f, Az, Bz);
-    constexpr float SLACK = 9.5367431640625e-07f; // 2^-20
+    constexpr float SLACK = SLAB_SLACK;
     const unsigned long long Bnxy = fma2(Sxy, pack2(-SLACK, -SLACK), B0xy), Bfxy = fma2(Sxy, pack2(SLACK, SLACK), B0xy);
     const float Bnz = __fmaf_rn(Sz, -SLACK, B0z), Bfz = __fmaf_rn(Sz, SLACK, B0z);
     float Bnx, Bny, Bfx, Bfy;
@@ -412,6 +428,83 @@ __device__ __forceinline__ bool node_step(const MeshRef &mr, const LocalRay &r, 
     return true;
 }
 
+// Node step of a ray that eight lanes trace together (lane c of the group
+// tests child c; the ray's state is the same in all eight). The steps of one
+// ray follow one another, so their latency, not their throughput, decides the
+// time of a launch with few rays and of every launch's last rays: testing the
+// children side by side takes a step's dependent instructions from about 200
+// to 60. Called by whole warps; `go`: this group's ray takes a step.
+// Arithmetic and results as node_step; false on a corrupt index.
+template <typename ST>
+__device__ __forceinline__ bool node_step_coop(bool go, const MeshRef &mr, const LocalRay &r, float best_t, uint32_t &ng_base,
+                                               uint32_t &ng_bits, uint32_t &tg_base, uint32_t &tg_bits, ST &st, uint32_t &visits,
+                                               uint32_t &err) {
+    const uint32_t lane = threadIdx.x & 31u, c = lane & 7u;
+    bool ok = true, hit = false;
+    uint32_t imask = 0, child_base = 0, tri_base = 0, meta_lo = 0, meta_hi = 0;
+    if (go) {
+        const uint32_t j = __ffs(ng_bits >> 24) - 1;
+        ng_bits &= ~(1u << (24 + j));
+        const uint32_t s = (j ^ r.oct) & 7u;
+        const uint32_t ni = ng_base + __popc((ng_bits & 0xFFu) & ((1u << s) - 1u));
+        if (ng_bits > 0x00FFFFFFu && !st.push_group(make_uint2(ng_base, ng_bits), c == 0)) {
+            err |= TRACE_ERR_STACK;
+            ok = false;
+        } else if (ni >= mr.node_count || ++visits > mr.node_count) {
+            err |= (ni >= mr.node_count) ? TRACE_ERR_BOUNDS : TRACE_ERR_LIMIT;
+            ok = false;
+        } else {
+            const WideNode *nd = mr.nodes + ni;
+            const uint4 w0 = __ldg(reinterpret_cast<const uint4 *>(nd)), w1 = __ldg(reinterpret_cast<const uint4 *>(nd) + 1);
+            const uint8_t *q = reinterpret_cast<const uint8_t *>(nd) + 32 + c; // qlo[axis][c] at 8 axis, qhi 24 further
+            const uint32_t lx = __ldg(q), ly = __ldg(q + 8), lz = __ldg(q + 16), hx = __ldg(q + 24), hy = __ldg(q + 32), hz = __ldg(q + 40);
+            imask = w0.w >> 24;
+            child_base = w1.x;
+            tri_base = w1.y;
+            meta_lo = w1.z;
+            meta_hi = w1.w;
+            float tn[3], tf[3];
+#pragma unroll
+            for (int a = 0; a < 3; a++) { // as node_step
+                const float p = __uint_as_float(a == 0 ? w0.x : (a == 1 ? w0.y : w0.z));
+                const float sc = __uint_as_float(((w0.w >> (8 * a)) & 0xFFu) << 23);
+                const float inv = a == 0 ? r.ix : (a == 1 ? r.iy : r.iz), o = a == 0 ? r.ox : (a == 1 ? r.oy : r.oz);
+                const uint32_t lo = a == 0 ? lx : (a == 1 ? ly : lz), hi = a == 0 ? hx : (a == 1 ? hy : hz);
+                const bool neg = (r.oct >> a) & 1u;
+                const float A = __fmul_rn(sc, inv), B = __fmul_rn(__fsub_rn(p, o), inv);
+                const float S = __fmaf_rn(fabsf(A), 33024.0f, fabsf(B)), B0 = __fmaf_rn(-32768.0f, A, B);
+                tn[a] = __fmaf_rn(__uint_as_float(0x47000000u | ((neg ? hi : lo) << 8)), A, __fmaf_rn(S, -SLAB_SLACK, B0));
+                tf[a] = __fmaf_rn(__uint_as_float(0x47000000u | ((neg ? lo : hi) << 8)), A, __fmaf_rn(S, SLAB_SLACK, B0));
+                if ((r.oct >> (3 + a)) & 1u) { // zero_axis_children
+                    const float pl = __fmaf_rn((float)lo, sc, p), ph = __fmaf_rn((float)hi, sc, p);
+                    if (o < pl || o > ph) ok = false;
+                }
+            }
+            const float tmin = max3f(tn[0], tn[1], fmaxf(tn[2], 0.0f)), tmax = min3f(tf[0], tf[1], fminf(tf[2], best_t));
+            hit = ok && !(__float_as_int(__fsub_rn(tmax, tmin)) < 0);
+            ok = true;
+        }
+    }
+    const uint32_t hit8 = (__ballot_sync(0xffffffffu, hit) >> (lane & 24u)) & 0xFFu;
+    if (go && ok) {
+        uint32_t inner = hit8 & imask;
+        if (r.oct & 1u) inner = ((inner & 0x55u) << 1) | ((inner >> 1) & 0x55u);
+        if (r.oct & 2u) inner = ((inner & 0x33u) << 2) | ((inner >> 2) & 0x33u);
+        if (r.oct & 4u) inner = ((inner & 0x0Fu) << 4) | ((inner >> 4) & 0x0Fu);
+        uint32_t leaf = 0;
+        for (uint32_t lv = hit8 & ~imask; lv; lv &= lv - 1u) {
+            const uint32_t sl = __ffs(lv) - 1u;
+            const uint32_t meta = ((sl < 4u ? meta_lo : meta_hi) >> (8u * (sl & 3u))) & 0xFFu;
+            leaf |= (meta >> 5) << (meta & 31u);
+        }
+        ng_base = child_base;
+        ng_bits = (inner << 24) | imask;
+        tg_base = tri_base;
+        tg_bits = leaf & 0x00FFFFFFu;
+    }
+    return ok;
+}
+
 // The reference's triangle arithmetic (_IntersectTri, CoreRef.cpp:18-40) on
 // one precomputed record (t0, t1, t2) and a ray given by origin and
 // direction: true when the ray's line passes the edge tests; then
@@ -435,6 +528,27 @@ __device__ __forceinline__ bool tri_core(const float4 &t0, const float4 &t1, con
         return true;
     }
     return false;
+}
+
+// A triangle test of a group's lane against the ray's best hit so far: true
+// when it is the closer one (tri_test's rule), with its t, u, v and index.
+template <typename BEST>
+__device__ __forceinline__ bool tri_candidate(const MeshRef &mr, const LocalRay &r, uint32_t li, const BEST &best, uint32_t &err, float &t,
+                                              float &u, float &v, int &gp, bool &solid) {
+    if (li >= mr.tri_count) {
+        err |= TRACE_ERR_BOUNDS;
+        return false;
+    }
+    const float4 *tp = reinterpret_cast<const float4 *>(mr.tris + li);
+    const float4 t0 = __ldg(tp), t1 = __ldg(tp + 1), t2 = __ldg(tp + 2);
+    float rdet, dett, detu, detv;
+    if (!tri_core(t0, t1, t2, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, rdet, dett, detu, detv)) return false;
+    t = __fmul_rn(dett, rdet);
+    gp = (int)(mr.prim_base + __float_as_uint(t2.z));
+    u = __fmul_rn(detu, rdet);
+    v = __fmul_rn(detv, rdet);
+    solid = (__float_as_int(t1.y) & TRI_SOLID_BIT) != 0;
+    return t > 0.0f && (t < best.t || (t == best.t && best.prim >= 0 && gp <= best.prim && (gp < best.prim || mr.obj < best.obj_of())));
 }
 
 // One triangle test; updates best when it is the closer hit. With SOLID,
