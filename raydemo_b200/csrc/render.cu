@@ -545,19 +545,44 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     // light samples of RAY_MAT_PRINCIPLED vertices wait in d_shadow (count in counter [8])
     // for their shadow rays; the reference's own lights are traced inside the shading
     bool ref_lights = false, nee = false, principled_only = true;
+    uint32_t max_lights = 0;
     for (const FrameJob &J : jobs) {
         ref_lights = ref_lights || J.sc.n_lights > 0;
+        max_lights = std::max(max_lights, J.sc.n_lights);
         nee = nee || J.sc.n_area_lights > 0;
         principled_only = principled_only && J.sc.principled_only;
     }
-    ShadowQueue shadow{nullptr, nullptr, nullptr, nullptr};
-    if (nee || adj) {
-        if (!adj) RG_CUDA_TRY(rb->d_shadow.ensure(std::max<size_t>(total, 1) * sizeof(ShadowRec)));
-        RG_CUDA_TRY(rb->d_shadow_rays.ensure(std::max<size_t>(total, 1) * 2 * sizeof(float4)));
-        RG_CUDA_TRY(rb->d_shadow_job.ensure(std::max<size_t>(total, 1) * sizeof(uint32_t)));
+    // The reference's lights: their shadow rays join the queue for the
+    // persistent any-hit trace where every scene has at most MAX_QUEUED_LIGHTS
+    // of them (the queue holds that many rays per ray of the launch, 100 bytes
+    // each) and none has area lights (whose emission the shading adds to the
+    // same colour), else the shading kernel traces them. Measured on B200 (16
+    // scenes with one sun each, 4.7 Mpixel, 4 samples, 6 bounces): shading with
+    // the shadow rays traced inside 11.3 ms; queued 4.7 ms of shading, 1.6 of
+    // any-hit traces and 0.6 of light sums.
+    const LightMode lights = !ref_lights                                            ? LIGHTS_NONE
+                             : (adj || nee || max_lights > MAX_QUEUED_LIGHTS)       ? LIGHTS_TRACED
+                             : max_lights == 1                                      ? LIGHTS_QUEUED_1
+                                                                                    : LIGHTS_QUEUED;
+    const bool queued = lights >= LIGHTS_QUEUED_1;
+    const uint64_t per_ray = lights == LIGHTS_QUEUED ? max_lights : 1;
+    if (per_ray * total > 0xffffffffull) {
+        set_error("too many light samples in one launch");
+        return RAY_ERR_INVALID_ARG;
+    }
+    const uint32_t max_shadow = (uint32_t)(per_ray * total);
+    ShadowQueue shadow{nullptr, nullptr, nullptr, nullptr, nullptr};
+    if (nee || adj || queued) {
+        const size_t cap = std::max<size_t>(max_shadow, 1);
+        if (!adj) RG_CUDA_TRY(rb->d_shadow.ensure(cap * std::max(sizeof(ShadowRec), sizeof(LightVertexRec))));
+        RG_CUDA_TRY(rb->d_shadow_rays.ensure(cap * 2 * sizeof(float4)));
+        RG_CUDA_TRY(rb->d_shadow_job.ensure(cap * sizeof(uint32_t)));
+        if (queued) RG_CUDA_TRY(rb->d_shadow_terms.ensure(cap * sizeof(float4)));
+        RG_CUDA_TRY(rb->d_hits.ensure(cap * sizeof(float4)));
         shadow.recs = adj ? static_cast<void *>(adj->recs) : rb->d_shadow.p;
         shadow.rays = static_cast<float4 *>(rb->d_shadow_rays.p);
         shadow.job = static_cast<uint32_t *>(rb->d_shadow_job.p);
+        shadow.terms = static_cast<float4 *>(rb->d_shadow_terms.p);
     }
     for (int k = 0; k < 2; k++) RG_CUDA_TRY(rb->d_job[k].ensure(std::max<size_t>(total, 1) * sizeof(uint32_t)));
     uint32_t *cnt = static_cast<uint32_t *>(rb->d_counters.p);
@@ -634,19 +659,20 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
         // shadow rays and the colour of the unblocked ones
         auto shade = [&](int b, int in, int out) -> cudaError_t {
             cudaError_t e = cudaSuccess;
-            if (nee || adj) e = cudaMemsetAsync(shadow_cnt, 0, sizeof(uint32_t), st);
+            if (nee || adj || queued) e = cudaMemsetAsync(shadow_cnt, 0, sizeof(uint32_t), st);
             if (e != cudaSuccess) return e;
             if (adj)
                 e = launch_adjoint_shade(d_jobs, b, rays[in], pay[in], job[in], adj->state[in], hits, obj, cnt + in, total, rays[out], pay[out],
                                          job[out], adj->state[out], cnt + out, shadow, adj->args, err, st, ref_lights, principled_only);
             else
                 e = launch_shade_jobs(d_jobs, sample, b, rays[in], pay[in], job[in], hits, obj, cnt + in, total, rays[out], pay[out], job[out],
-                                      cnt + out, shadow, ref_lights, principled_only, err, ray_stats, st);
-            if (e != cudaSuccess || !(nee || adj)) return e;
-            e = launch_trace_closest(sv, shadow.rays, total, hits, nullptr, err, nullptr, false, st, tps);
+                                      cnt + out, shadow, max_shadow, lights, principled_only, err, ray_stats, st);
+            if (e != cudaSuccess || !(nee || adj || queued)) return e;
+            e = launch_trace_closest(sv, shadow.rays, max_shadow, hits, nullptr, err, nullptr, false, st, tps);
             if (e != cudaSuccess) return e;
             if (adj) return launch_adjoint_shadow_apply(d_jobs, b, shadow, hits, total, adj->state[out], adj->args, err, st);
-            return launch_shadow_apply(d_jobs, sample, b, shadow, hits, total, err, ray_stats, st);
+            if (queued) return launch_light_apply(d_jobs, sample, b, shadow, hits, max_shadow, err, ray_stats, st);
+            return launch_shadow_apply(d_jobs, sample, b, shadow, hits, max_shadow, err, ray_stats, st);
         };
         RG_CUDA_TRY(shade(2, 0, 1));
         if (ev) RG_CUDA_TRY(cudaEventRecord(ev[3], st));
@@ -689,7 +715,7 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     GraphKey key;
     key.add(d_jobs).add(n_jobs).add(total).add(sample0).add(samples).add(sort_mask).add(bounces).add(resolve).add(adj).add(st);
     for (int q = 0; q < 2; q++) key.add(rays[q]).add(pay[q]).add(job[q]);
-    key.add(hits).add(obj).add(cnt).add(shadow.recs).add(shadow.rays).add(shadow.job).add(rb->d_loop_sort.p).add(nee).add(ref_lights).add(principled_only);
+    key.add(hits).add(obj).add(cnt).add(shadow.recs).add(shadow.rays).add(shadow.job).add(shadow.terms).add(max_shadow).add(lights).add(rb->d_loop_sort.p).add(nee).add(ref_lights).add(principled_only);
     key.add(sv.nodes).add(sv.leaf_tris).add(sv.inst).add(sv.n_inst).add(tp.persistent).add(tp.refill_min).add(tp.max_depth).add(tp.views);
     key.add(sv.tlas).add(sv.tlas_inst).add(sv.tlas_count).add(tp.tlas).add(tp.block).add(tp.smem_stack).add(tp.one_tri);
     key.add(ev).add(geo_best).add(geo_tris).add(persp);

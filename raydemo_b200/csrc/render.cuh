@@ -189,15 +189,36 @@ struct ShadowRec {
 };
 static_assert(sizeof(ShadowRec) == 48, "shadow record layout");
 
-// Where a shading launch appends its light samples: the records (ShadowRec
-// or AdjShadowRec), their shadow rays (o, tmax = segment length; d) for the
-// any-hit trace, the rays' jobs, and the device count.
+// A diffuse vertex waiting for the shadow rays of the reference's lights (48
+// bytes, at the slot of its first ray): what its lights' sum is multiplied by
+// (albedo, path weight) on the way to temp[index] of job `job`.
+struct LightVertexRec {
+    float alb[3], rc[3];
+    uint32_t index, job, rand_index, pad[3];
+};
+static_assert(sizeof(LightVertexRec) == 48, "light vertex record layout");
+
+// Where a shading launch appends its light samples: the records (ShadowRec,
+// LightVertexRec or AdjShadowRec), their shadow rays (o, tmax = segment
+// length; d) for the any-hit trace, the rays' jobs, and the device count.
+// terms (LightVertexRec only, one per ray): the light's contribution when
+// unblocked, and its index with the vertex's ray count above it (LIGHT_COUNT_
+// SHIFT; 0 on all but the vertex's first ray).
 struct ShadowQueue {
     void *recs;
     float4 *rays;
     uint32_t *job;
     uint32_t *count;
+    float4 *terms;
 };
+constexpr uint32_t LIGHT_COUNT_SHIFT = 8;
+
+// How a shading launch treats the reference's point, spot and directional
+// lights: the scenes have none; their shadow rays are traced in the shading
+// kernel; or they go to the shadow queue, up to one or MAX_QUEUED_LIGHTS per
+// vertex, for the persistent any-hit trace.
+enum LightMode { LIGHTS_NONE = 0, LIGHTS_TRACED = 1, LIGHTS_QUEUED_1 = 2, LIGHTS_QUEUED = 3 };
+constexpr uint32_t MAX_QUEUED_LIGHTS = 4;
 
 // ---- the path-replay adjoint (differentiable parameters of RAY_MAT_PRINCIPLED)
 constexpr int ADJ_MAX_SLOTS = 64; // roughness slots
@@ -254,18 +275,22 @@ cudaError_t launch_geo_rays(const FrameJob *jobs, int n_jobs, uint32_t total, in
 // Shades the hits of *in_count rays (bounce: pass_info_t::bounce, 2 for the
 // primary rays: SetPixel, else AddPixel with alpha 0), appends the rays that
 // go on to out (count *out_count) and the light samples of RAY_MAT_PRINCIPLED
-// vertices to shadow (count *shadow_count, zeroed beforehand). ref_lights:
-// some job's scene has the reference's lights (traced inside the shading).
+// vertices to shadow (count *shadow_count, zeroed beforehand). lights: what
+// happens to the reference's lights (LightMode); max_shadow: the queue's size.
 cudaError_t launch_shade_jobs(const FrameJob *jobs, int sample, int bounce, const float4 *rays, const RayPayload *pay, const uint32_t *ray_job,
                               const float4 *hits, const int32_t *obj, const uint32_t *in_count, uint32_t max_rays, float4 *out_rays,
-                              RayPayload *out_pay, uint32_t *out_job, uint32_t *out_count, const ShadowQueue &shadow, bool ref_lights,
-                              bool principled_only, uint32_t *err, unsigned long long *ray_stats, cudaStream_t st);
+                              RayPayload *out_pay, uint32_t *out_job, uint32_t *out_count, const ShadowQueue &shadow, uint32_t max_shadow,
+                              LightMode lights, bool principled_only, uint32_t *err, unsigned long long *ray_stats, cudaStream_t st);
 // After the any-hit trace of a shading launch's shadow rays (hits): adds the
 // colour of each unblocked light sample to its pixel. A ray whose first hit
 // is on a non-solid triangle takes the full visibility walk through the
 // transparent layers (ComputeVisibility) instead.
 cudaError_t launch_shadow_apply(const FrameJob *jobs, int sample, int bounce, const ShadowQueue &shadow, const float4 *hits, uint32_t max_recs,
                                 uint32_t *err, unsigned long long *ray_stats, cudaStream_t st);
+// The same for the reference's queued lights: sums each diffuse vertex's
+// unblocked lights in their order, times albedo and path weight, into its pixel.
+cudaError_t launch_light_apply(const FrameJob *jobs, int sample, int bounce, const ShadowQueue &shadow, const float4 *hits, uint32_t max_recs,
+                               uint32_t *err, unsigned long long *ray_stats, cudaStream_t st);
 // clean += (temp - clean) / iteration over every job's rect, then final = tone(clean)
 cudaError_t launch_resolve_jobs(const FrameJob *jobs, int n_jobs, uint32_t total, int sample, cudaStream_t st);
 // The whole frame of every job in one launch (ray generation, all bounces,

@@ -247,11 +247,15 @@ __device__ float compute_visibility(const RenderScene &sc, V3 p1, V3 p2, const f
     return visibility;
 }
 
-// AcumulateLightContribution, CoreRef.cpp:1898-1933
-// dcol (may be null): also adds the contribution's derivative by sigma.
-__device__ __forceinline__ void accumulate_light(const RenderScene &sc, const LightRec &l, V3 I, V3 P, V3 N, V3 B, V3 plane_N, float sigma,
-                                                 const float *halton, int hi, int rand_hash2, float rand_offset, float rand_offset2, V3 &col,
-                                                 Stack<true> &st, uint32_t &err, uint32_t &nshadow, V3 *dcol = nullptr) {
+// AcumulateLightContribution (CoreRef.cpp:1898-1933) up to its shadow ray:
+// false when the light adds nothing; else the factors of its contribution,
+// which is (color * dot1) * visibility * atten * brdf for the direction L.
+struct LightTerm {
+    V3 L;
+    float dot1, atten;
+};
+__device__ __forceinline__ bool light_term(const LightRec &l, V3 P, V3 N, V3 B, const float *halton, int hi, float rand_offset,
+                                           float rand_offset2, LightTerm &lt) {
     const V3 lpos = v3(l.pos);
     V3 L = P - lpos;
     const float distance = length(L);
@@ -271,18 +275,39 @@ __device__ __forceinline__ void accumulate_light(const RenderScene &sc, const Li
     atten = fmax_std(atten, 0.0f);
     const float dot1 = fmax_std(dot(L, N), 0.0f);
     const float dot2 = dot(L, v3(l.dir));
-    if (dot1 > FLT_EPS_ && dot2 > l.spot && (l.brightness * atten) > FLT_EPS_) {
-        const float visibility = compute_visibility(sc, P + HIT_BIAS * plane_N, lpos, halton, hi, rand_hash2, st, err, nshadow);
-        if (dcol) {
-            float d_sigma = 0.0f;
-            const float on = brdf_oren_nayar_d(L, I, N, B, sigma, d_sigma);
-            col = col + v3(l.col) * dot1 * visibility * atten * on;
-            *dcol = *dcol + v3(l.col) * dot1 * visibility * atten * d_sigma;
-        } else {
-            col = col + v3(l.col) * dot1 * visibility * atten * brdf_oren_nayar(L, I, N, B, sigma);
-        }
+    lt.L = L;
+    lt.dot1 = dot1;
+    lt.atten = atten;
+    return dot1 > FLT_EPS_ && dot2 > l.spot && (l.brightness * atten) > FLT_EPS_;
+}
+
+// The light's contribution, its shadow ray traced here.
+// dcol (may be null): also adds the contribution's derivative by sigma.
+__device__ __forceinline__ void accumulate_light(const RenderScene &sc, const LightRec &l, V3 I, V3 P, V3 N, V3 B, V3 plane_N, float sigma,
+                                                 const float *halton, int hi, int rand_hash2, float rand_offset, float rand_offset2, V3 &col,
+                                                 Stack<true> &st, uint32_t &err, uint32_t &nshadow, V3 *dcol = nullptr) {
+    LightTerm lt;
+    if (!light_term(l, P, N, B, halton, hi, rand_offset, rand_offset2, lt)) return;
+    const float visibility = compute_visibility(sc, P + HIT_BIAS * plane_N, v3(l.pos), halton, hi, rand_hash2, st, err, nshadow);
+    if (dcol) {
+        float d_sigma = 0.0f;
+        const float on = brdf_oren_nayar_d(lt.L, I, N, B, sigma, d_sigma);
+        col = col + v3(l.col) * lt.dot1 * visibility * lt.atten * on;
+        *dcol = *dcol + v3(l.col) * lt.dot1 * visibility * lt.atten * d_sigma;
+    } else {
+        col = col + v3(l.col) * lt.dot1 * visibility * lt.atten * brdf_oren_nayar(lt.L, I, N, B, sigma);
     }
 }
+
+// A diffuse vertex's queued lights (bit k of mask: light k has a shadow ray
+// from o, and contributes t[k] when unblocked), with what their sum is
+// multiplied by: the pixel takes rc * ((sum of t) * alb), as shade_hit's
+// colour of a vertex whose lights are traced in place.
+template <int NL>
+struct LightReq {
+    V3 t[NL], o, alb, rc;
+    uint32_t mask;
+};
 
 struct NewRay {
     float4 r0, r1;
@@ -356,14 +381,15 @@ __device__ __forceinline__ void set3(float *dst, V3 v) {
 
 // ShadeSurface, CoreRef.cpp:2055-2391. Returns the pixel contribution;
 // fills nr and sets emit when the path continues, and sr with a
-// RAY_MAT_PRINCIPLED vertex's light sample. REF_LIGHTS: the scene may have
-// the reference's point/spot/directional lights (their shadow rays are traced
-// here); without, the kernel carries no traversal code.
-template <bool REF_LIGHTS, bool PONLY = false>
+// RAY_MAT_PRINCIPLED vertex's light sample. LIGHTS: the scene may have the
+// reference's point/spot/directional lights, traced here or put into lq (a
+// LightReq; LightMode); without LIGHTS_TRACED the kernel carries no traversal code.
+template <int LIGHTS, bool PONLY = false, int NL = 1>
 __device__ F4 shade_hit(const RenderScene &sc, const PassInfo &pi, int rand_index, const float *halton, float4 hit, int obj,
                         float4 r0, float4 r1, const RayPayload &ray, NewRay &nr, bool &emit, ShadowReq &sr, Stack<true> &st,
-                        uint32_t &err, uint32_t &nshadow, VertexGrad *vg = nullptr) {
+                        uint32_t &err, uint32_t &nshadow, VertexGrad *vg = nullptr, LightReq<NL> *lq = nullptr) {
     emit = false;
+    if (LIGHTS >= LIGHTS_QUEUED_1) lq->mask = 0;
     sr.valid = false;
     if (vg) vg->valid = vg->diffuse = false;
     const int prim = __float_as_int(hit.x);
@@ -520,7 +546,20 @@ __device__ F4 shade_hit(const RenderScene &sc, const PassInfo &pi, int rand_inde
         const bool dgrad = vg && vg->diffuse;
         if (dgrad) vg->albedo_on = consider_albedo;
         if (!(pi.flags & PASS_SKIP_DIRECT) || pi.bounce > 2) {
-            if (REF_LIGHTS)
+            if (LIGHTS >= LIGHTS_QUEUED_1) {
+#pragma unroll
+                for (uint32_t li = 0; li < (uint32_t)NL; li++) {
+                    if (li >= sc.n_lights) break;
+                    const LightRec &l = sc.lights[li];
+                    LightTerm lt;
+                    if (!light_term(l, P, N, B, halton, hi, rand_offset, rand_offset2, lt)) continue;
+                    lq->t[li] = v3(l.col) * lt.dot1 * lt.atten * brdf_oren_nayar(lt.L, I, N, B, sigma_d);
+                    lq->mask |= 1u << li;
+                }
+                lq->o = P + HIT_BIAS * plane_N;
+                lq->alb = consider_albedo ? alb : v3(1.0f, 1.0f, 1.0f);
+                lq->rc = v3(ray.c);
+            } else if (LIGHTS == LIGHTS_TRACED)
                 for (uint32_t li = 0; li < sc.n_lights; li++)
                     accumulate_light(sc, sc.lights[li], I, P, N, B, plane_N, sigma_d, halton, hi, rand_hash2, rand_offset, rand_offset2, col, st,
                                      err, nshadow, dgrad ? &vg->d_direct : nullptr);
@@ -788,12 +827,13 @@ __device__ F4 shade_hit(const RenderScene &sc, const PassInfo &pi, int rand_inde
 // the hit: weight 1 for rays whose last vertex did not sample quad lights
 // (pdf 0 in the payload), else the power heuristic against the light pdf that
 // next-event estimation at that vertex used.
-template <bool REF_LIGHTS, bool PONLY = false>
+template <int LIGHTS, bool PONLY = false, int NL = 1>
 __device__ __forceinline__ F4 shade_surface(const RenderScene &sc, const PassInfo &pi, int rand_index, const float *halton, float4 hit,
                                             int obj, float4 r0, float4 r1, const RayPayload &ray, NewRay &nr, bool &emit, ShadowReq &sr,
-                                            Stack<true> &st, uint32_t &err, uint32_t &nshadow, VertexGrad *vg = nullptr) {
-    F4 c = shade_hit<REF_LIGHTS, PONLY>(sc, pi, rand_index, halton, hit, obj, r0, r1, ray, nr, emit, sr, st, err, nshadow, vg);
-    if (sc.n_area_lights == 0) return c;
+                                            Stack<true> &st, uint32_t &err, uint32_t &nshadow, VertexGrad *vg = nullptr,
+                                            LightReq<NL> *lq = nullptr) {
+    F4 c = shade_hit<LIGHTS, PONLY, NL>(sc, pi, rand_index, halton, hit, obj, r0, r1, ray, nr, emit, sr, st, err, nshadow, vg, lq);
+    if (LIGHTS >= LIGHTS_QUEUED_1 || sc.n_area_lights == 0) return c; // (lights are queued in scenes without area lights only)
     const V3 o = v3(r0.x, r0.y, r0.z), d = v3(r1.x, r1.y, r1.z);
     const float tmax = __float_as_int(hit.x) >= 0 ? hit.y : MAX_DIST;
     const float prev_pdf = __uint_as_float(ray.pad[0]);
@@ -1061,19 +1101,20 @@ __global__ void k_geo_rays(const FrameJob *__restrict__ jobs, int n_jobs, uint32
 // with alpha 0. A continuation ray is appended where the path goes on and its
 // job traces another bounce. PONLY: every material of every job's scene is
 // RAY_MAT_PRINCIPLED (and no scene has the reference's lights), so the
-// kernel carries none of the other materials' code.
-template <bool PRIMARY, bool REF_LIGHTS, bool PONLY = false>
-__global__ void __launch_bounds__(SHADE_BLOCK, REF_LIGHTS ? 3 : 4) k_shade_jobs(const FrameJob *__restrict__ jobs, int sample, int bounce,
+// kernel carries none of the other materials' code. LIGHTS: LightMode.
+template <bool PRIMARY, int LIGHTS, bool PONLY = false>
+__global__ void __launch_bounds__(SHADE_BLOCK, LIGHTS == LIGHTS_TRACED ? 3 : 4) k_shade_jobs(const FrameJob *__restrict__ jobs, int sample, int bounce,
                                                             const float4 *__restrict__ rays, const RayPayload *__restrict__ pay,
                                                             const uint32_t *__restrict__ ray_job, const float4 *__restrict__ hits,
                                                             const int32_t *__restrict__ obj, const uint32_t *__restrict__ in_count,
                                                             uint32_t max_rays, float4 *__restrict__ out_rays, RayPayload *__restrict__ out_pay,
                                                             uint32_t *__restrict__ out_job, uint32_t *__restrict__ out_count,
-                                                            ShadowQueue shadow, uint32_t *__restrict__ err_out,
+                                                            ShadowQueue shadow, uint32_t max_shadow, uint32_t *__restrict__ err_out,
                                                             unsigned long long *__restrict__ ray_stats) {
-    __shared__ uint2 s_stack[REF_LIGHTS ? trav::SMEM_STACK * SHADE_BLOCK : 1];
+    __shared__ uint2 s_stack[LIGHTS == LIGHTS_TRACED ? trav::SMEM_STACK * SHADE_BLOCK : 1];
+    constexpr int NL = LIGHTS == LIGHTS_QUEUED ? (int)MAX_QUEUED_LIGHTS : 1;
     Stack<true> st;
-    st.smem = s_stack + threadIdx.x;
+    st.smem = s_stack + (LIGHTS == LIGHTS_TRACED ? threadIdx.x : 0);
     st.sp = 0;
     uint32_t err = 0, nshadow = 0;
     const uint32_t n = min(*in_count, max_rays);
@@ -1085,6 +1126,8 @@ __global__ void __launch_bounds__(SHADE_BLOCK, REF_LIGHTS ? 3 : 4) k_shade_jobs(
         NewRay nr;
         ShadowReq sr;
         sr.valid = false;
+        LightReq<NL> lq;
+        lq.mask = 0;
         uint32_t sr_index = 0, sr_rand = 0;
         if (i < n) {
             j = ray_job[i];
@@ -1099,8 +1142,8 @@ __global__ void __launch_bounds__(SHADE_BLOCK, REF_LIGHTS ? 3 : 4) k_shade_jobs(
             pi.bounce = bounce;
             const int rand_index = (pi.flags & PASS_COHERENT) ? c_sampling_pattern[(y % 8) * 8 + (x % 8)] : index;
             bool emit = false;
-            const F4 c = shade_surface<REF_LIGHTS, PONLY>(J.sc, pi, rand_index, J.halton, hits[i], obj[i], r0, r1, p, nr, emit, sr, st, err,
-                                                          nshadow);
+            const F4 c = shade_surface<LIGHTS, PONLY, NL>(J.sc, pi, rand_index, J.halton, hits[i], obj[i], r0, r1, p, nr, emit, sr, st, err,
+                                                          nshadow, nullptr, &lq);
             sr_index = (uint32_t)index;
             sr_rand = (uint32_t)rand_index;
             append = emit && bounce - 2 < J.bounces;
@@ -1128,14 +1171,51 @@ __global__ void __launch_bounds__(SHADE_BLOCK, REF_LIGHTS ? 3 : 4) k_shade_jobs(
                 J.temp[index] = acc;
             }
         }
+        if (LIGHTS >= LIGHTS_QUEUED_1) {
+            // append of the queued lights: consecutive slots per vertex
+            const uint32_t cnt = (uint32_t)__popc(lq.mask);
+            uint32_t incl = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= (uint32_t)o) incl += y;
+            }
+            uint32_t slot = 0;
+            if (lane == 31u && incl) slot = atomicAdd(shadow.count, incl);
+            slot = __shfl_sync(0xffffffffu, slot, 31) + incl - cnt;
+            if (cnt && slot + cnt <= max_shadow) {
+                LightVertexRec rec;
+                rec.alb[0] = lq.alb.x; rec.alb[1] = lq.alb.y; rec.alb[2] = lq.alb.z;
+                rec.rc[0] = lq.rc.x; rec.rc[1] = lq.rc.y; rec.rc[2] = lq.rc.z;
+                rec.index = sr_index;
+                rec.job = j;
+                rec.rand_index = sr_rand;
+                rec.pad[0] = rec.pad[1] = rec.pad[2] = 0;
+                static_cast<LightVertexRec *>(shadow.recs)[slot] = rec;
+                uint32_t head = cnt << LIGHT_COUNT_SHIFT;
+                const LightRec *lights = jobs[j].sc.lights;
+#pragma unroll
+                for (uint32_t li = 0; li < (uint32_t)NL; li++) {
+                    if (!((lq.mask >> li) & 1u)) continue;
+                    float4 q0, q1;
+                    shadow_ray(lq.o, v3(lights[li].pos), q0, q1);
+                    shadow.rays[2ull * slot] = q0;
+                    shadow.rays[2ull * slot + 1] = q1;
+                    shadow.job[slot] = j;
+                    shadow.terms[slot] = make_float4(lq.t[li].x, lq.t[li].y, lq.t[li].z, __uint_as_float(li | head));
+                    head = 0;
+                    slot++;
+                }
+            }
+        }
         // warp-aggregated append of the light samples
-        const uint32_t ms = __ballot_sync(0xffffffffu, sr.valid);
+        const uint32_t ms = LIGHTS >= LIGHTS_QUEUED_1 ? 0u : __ballot_sync(0xffffffffu, sr.valid);
         if (ms) {
             uint32_t slot = 0;
             const uint32_t leader = __ffs(ms) - 1;
             if (lane == leader) slot = atomicAdd(shadow.count, (uint32_t)__popc(ms));
             slot = __shfl_sync(0xffffffffu, slot, leader) + __popc(ms & ((1u << lane) - 1u));
-            if (sr.valid && slot < max_rays) {
+            if (sr.valid && slot < max_shadow) {
                 ShadowRec rec;
                 rec.o[0] = sr.o.x; rec.o[1] = sr.o.y; rec.o[2] = sr.o.z;
                 rec.p2[0] = sr.p2.x; rec.p2[1] = sr.p2.y; rec.p2[2] = sr.p2.z;
@@ -1224,6 +1304,53 @@ __global__ void __launch_bounds__(SHADE_BLOCK) k_shadow_apply(const FrameJob *__
     }
 }
 
+// Adds each diffuse vertex's queued lights to its pixel: the sum of the
+// unblocked ones in light order, times the albedo, times the path weight -- the
+// products and sums, in their order, of a vertex whose lights are traced in
+// place, whose pixel takes that colour as the shading's (queued lights go with
+// scenes without area lights, where it is the whole colour of the vertex). A
+// blocked light adds its term times zero.
+__global__ void __launch_bounds__(SHADE_BLOCK) k_light_apply(const FrameJob *__restrict__ jobs, int sample, int bounce, ShadowQueue q,
+                                                             const float4 *__restrict__ hits, uint32_t max_recs,
+                                                             uint32_t *__restrict__ err_out, unsigned long long *__restrict__ ray_stats) {
+    __shared__ uint2 s_stack[trav::SMEM_STACK * SHADE_BLOCK];
+    Stack<true> st;
+    st.smem = s_stack + threadIdx.x;
+    st.sp = 0;
+    uint32_t err = 0, nshadow = 0;
+    const uint32_t n = min(*q.count, max_recs);
+    const LightVertexRec *recs = static_cast<const LightVertexRec *>(q.recs);
+    for (uint32_t i = blockIdx.x * SHADE_BLOCK + threadIdx.x; i < n; i += gridDim.x * SHADE_BLOCK) {
+        const float4 first = q.terms[i];
+        const uint32_t cnt = __float_as_uint(first.w) >> LIGHT_COUNT_SHIFT;
+        if (cnt == 0 || cnt > n - i) continue; // not a vertex's first ray
+        const LightVertexRec rec = recs[i];
+        const FrameJob &J = jobs[rec.job];
+        V3 col = v3(0.0f, 0.0f, 0.0f);
+        for (uint32_t k = 0; k < cnt; k++) {
+            const float4 t = k == 0 ? first : q.terms[i + k];
+            const uint32_t li = __float_as_uint(t.w) & ((1u << LIGHT_COUNT_SHIFT) - 1u);
+            const float4 r0 = q.rays[2ull * (i + k)];
+            const float o[3] = {r0.x, r0.y, r0.z};
+            const bool vis = sample_visible(J, J.pi.iteration + sample, bounce, o, J.sc.lights[li].pos, rec.rand_index, hits[i + k], st, err,
+                                            nshadow);
+            const V3 term = v3(t.x, t.y, t.z);
+            col = col + (vis ? term : term * 0.0f);
+        }
+        col = col * v3(rec.alb);
+        float4 acc = J.temp[rec.index];
+        acc.x += rec.rc[0] * col.x;
+        acc.y += rec.rc[1] * col.y;
+        acc.z += rec.rc[2] * col.z;
+        J.temp[rec.index] = acc;
+    }
+    if (err) atomicOr(err_out, err);
+    if (ray_stats) {
+        const uint32_t ws = __reduce_add_sync(0xffffffffu, nshadow);
+        if ((threadIdx.x & 31u) == 0 && ws) atomicAdd(&ray_stats[1], (unsigned long long)ws);
+    }
+}
+
 // Accumulation and tone of every job's rect, one thread per pixel.
 __global__ void k_resolve_jobs(const FrameJob *__restrict__ jobs, int n_jobs, uint32_t total, int sample) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1264,7 +1391,7 @@ __device__ __forceinline__ void render_path(const FrameJob &J, uint32_t i, int i
     bool emit = false;
     ShadowReq sr;
     const int rand_hash2 = hash_i(hash_i(rand_index));
-    F4 c = shade_surface<true>(J.sc, pi, rand_index, J.halton,
+    F4 c = shade_surface<LIGHTS_TRACED>(J.sc, pi, rand_index, J.halton,
                                make_float4(__int_as_float(b.prim), b.t, b.prim >= 0 ? b.u : 0.0f, b.prim >= 0 ? b.v : 0.0f), b.obj, r0, r1, pay,
                                nr, emit, sr, st, err, nshadow);
     float4 acc = make_float4(c.x, c.y, c.z, c.w);
@@ -1296,7 +1423,7 @@ __device__ __forceinline__ void render_path(const FrameJob &J, uint32_t i, int i
         b = trace_closest_scene(J.sc.sv, r0, r1, st, err);
         nrays++;
         pi.bounce = bounce + 3;
-        c = shade_surface<true>(J.sc, pi, rand_index, J.halton,
+        c = shade_surface<LIGHTS_TRACED>(J.sc, pi, rand_index, J.halton,
                                 make_float4(__int_as_float(b.prim), b.t, b.prim >= 0 ? b.u : 0.0f, b.prim >= 0 ? b.v : 0.0f), b.obj, r0, r1,
                                 pay, nr, emit, sr, st, err, nshadow);
         acc.x += c.x;
@@ -1483,7 +1610,7 @@ __global__ void __launch_bounds__(SHADE_BLOCK, 3) k_adjoint_shade(const FrameJob
             const int rand_index = (pi.flags & PASS_COHERENT) ? c_sampling_pattern[(y % 8) * 8 + (x % 8)] : index;
             bool emit = false;
             VertexGrad vg;
-            const F4 c = shade_surface<REF_LIGHTS, PONLY>(sc, pi, rand_index, J.halton, hits[i], obj[i], r0, r1, p, nr, emit, sr, st, err,
+            const F4 c = shade_surface<REF_LIGHTS ? LIGHTS_TRACED : LIGHTS_NONE, PONLY>(sc, pi, rand_index, J.halton, hits[i], obj[i], r0, r1, p, nr, emit, sr, st, err,
                                                           nshadow, &vg);
             // the sum as the sample buffer takes it (SetPixel on camera rays, AddPixel after)
             if (PRIMARY) {
@@ -1708,29 +1835,47 @@ static int resident_blocks(K kernel, int fallback_per_sm) {
 
 cudaError_t launch_shade_jobs(const FrameJob *jobs, int sample, int bounce, const float4 *rays, const RayPayload *pay, const uint32_t *ray_job,
                               const float4 *hits, const int32_t *obj, const uint32_t *in_count, uint32_t max_rays, float4 *out_rays,
-                              RayPayload *out_pay, uint32_t *out_job, uint32_t *out_count, const ShadowQueue &shadow, bool ref_lights,
-                              bool principled_only, uint32_t *err, unsigned long long *ray_stats, cudaStream_t st) {
-    const bool ponly = principled_only && !ref_lights;
-    static int resident[3] = {0, 0, 0};
-    int &res = resident[ref_lights ? 1 : (ponly ? 2 : 0)];
+                              RayPayload *out_pay, uint32_t *out_job, uint32_t *out_count, const ShadowQueue &shadow, uint32_t max_shadow,
+                              LightMode lights, bool principled_only, uint32_t *err, unsigned long long *ray_stats, cudaStream_t st) {
+    const bool ponly = principled_only && lights == LIGHTS_NONE;
+    static int resident[5] = {0, 0, 0, 0, 0};
+    int &res = resident[ponly ? 4 : (int)lights];
     if (res == 0)
-        res = ref_lights ? resident_blocks(k_shade_jobs<false, true>, 4)
-                         : (ponly ? resident_blocks(k_shade_jobs<false, false, true>, 4) : resident_blocks(k_shade_jobs<false, false>, 4));
+        res = ponly                       ? resident_blocks(k_shade_jobs<false, LIGHTS_NONE, true>, 4)
+              : lights == LIGHTS_NONE     ? resident_blocks(k_shade_jobs<false, LIGHTS_NONE>, 4)
+              : lights == LIGHTS_TRACED   ? resident_blocks(k_shade_jobs<false, LIGHTS_TRACED>, 3)
+              : lights == LIGHTS_QUEUED_1 ? resident_blocks(k_shade_jobs<false, LIGHTS_QUEUED_1>, 4)
+                                          : resident_blocks(k_shade_jobs<false, LIGHTS_QUEUED>, 4);
     const uint32_t need = (max_rays + SHADE_BLOCK - 1) / SHADE_BLOCK;
     const uint32_t blocks = need < (uint32_t)res ? (need > 0 ? need : 1) : (uint32_t)res;
-#define RG_SHADE(P, R, O)                                                                                                                  \
-    k_shade_jobs<P, R, O><<<blocks, SHADE_BLOCK, 0, st>>>(jobs, sample, bounce, rays, pay, ray_job, hits, obj, in_count, max_rays, out_rays, \
-                                                          out_pay, out_job, out_count, shadow, err, ray_stats)
-    if (bounce == 2) {
-        if (ref_lights) RG_SHADE(true, true, false);
-        else if (ponly) RG_SHADE(true, false, true);
-        else RG_SHADE(true, false, false);
-    } else {
-        if (ref_lights) RG_SHADE(false, true, false);
-        else if (ponly) RG_SHADE(false, false, true);
-        else RG_SHADE(false, false, false);
-    }
+#define RG_SHADE(L, O)                                                                                                                     \
+    do {                                                                                                                                   \
+        if (bounce == 2)                                                                                                                   \
+            k_shade_jobs<true, L, O><<<blocks, SHADE_BLOCK, 0, st>>>(jobs, sample, bounce, rays, pay, ray_job, hits, obj, in_count,         \
+                                                                     max_rays, out_rays, out_pay, out_job, out_count, shadow, max_shadow,  \
+                                                                     err, ray_stats);                                                      \
+        else                                                                                                                               \
+            k_shade_jobs<false, L, O><<<blocks, SHADE_BLOCK, 0, st>>>(jobs, sample, bounce, rays, pay, ray_job, hits, obj, in_count,        \
+                                                                      max_rays, out_rays, out_pay, out_job, out_count, shadow, max_shadow, \
+                                                                      err, ray_stats);                                                     \
+    } while (0)
+    if (ponly) RG_SHADE(LIGHTS_NONE, true);
+    else if (lights == LIGHTS_NONE) RG_SHADE(LIGHTS_NONE, false);
+    else if (lights == LIGHTS_TRACED) RG_SHADE(LIGHTS_TRACED, false);
+    else if (lights == LIGHTS_QUEUED_1) RG_SHADE(LIGHTS_QUEUED_1, false);
+    else RG_SHADE(LIGHTS_QUEUED, false);
 #undef RG_SHADE
+    return cudaGetLastError();
+}
+
+cudaError_t launch_light_apply(const FrameJob *jobs, int sample, int bounce, const ShadowQueue &shadow, const float4 *hits, uint32_t max_recs,
+                               uint32_t *err, unsigned long long *ray_stats, cudaStream_t st) {
+    static int resident = 0;
+    if (resident == 0) resident = resident_blocks(k_light_apply, 4);
+    if (max_recs == 0) return cudaSuccess;
+    const uint32_t need = (max_recs + SHADE_BLOCK - 1) / SHADE_BLOCK;
+    const uint32_t blocks = need < (uint32_t)resident ? need : (uint32_t)resident;
+    k_light_apply<<<blocks, SHADE_BLOCK, 0, st>>>(jobs, sample, bounce, shadow, hits, max_recs, err, ray_stats);
     return cudaGetLastError();
 }
 
