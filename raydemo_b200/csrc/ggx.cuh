@@ -40,12 +40,17 @@ __device__ __forceinline__ uint32_t nested_scramble(uint32_t x, uint32_t seed) {
     return __brev(x);
 }
 
-// Second Sobol dimension: generator matrix = Pascal's triangle mod 2.
+// Second Sobol dimension: generator matrix = Pascal's triangle mod 2, entry
+// (k, i) being C(i, k) mod 2, which is 1 exactly when k's bits are a subset of
+// i's (Lucas). So the product is the XOR over supersets, one step per bit of
+// the bit numbers, in place of a step per bit of the index.
 __device__ __forceinline__ uint32_t sobol_dim1(uint32_t i) {
-    uint32_t r = 0, v = 0x80000000u;
-    for (; i; i >>= 1, v ^= v >> 1)
-        if (i & 1u) r ^= v;
-    return r;
+    i ^= (i >> 1) & 0x55555555u;
+    i ^= (i >> 2) & 0x33333333u;
+    i ^= (i >> 4) & 0x0F0F0F0Fu;
+    i ^= (i >> 8) & 0x00FF00FFu;
+    i ^= i >> 16;
+    return __brev(i);
 }
 
 // Sample `index` of the scrambled 2D sequence of a (pixel, dimension pair) seed, in [0, 1)^2.
@@ -138,8 +143,10 @@ __device__ __forceinline__ bool sample(const Params &p, V3 wo, float u1, float u
         const V3 t2 = cross(vh, t1);
         const float r = sqrtf(u1);
         const float phi = 2.0f * PI_G * u2;
-        const float q1 = r * cr_cos(phi);
-        float q2 = r * cr_sin(phi);
+        float sin_phi, cos_phi;
+        cr_sincos(phi, sin_phi, cos_phi);
+        const float q1 = r * cos_phi;
+        float q2 = r * sin_phi;
         const float s = 0.5f * (1.0f + vh.z);
         q2 = (1.0f - s) * sqrtf(1.0f - q1 * q1) + s * q2;
         const V3 nh = t1 * q1 + t2 * q2 + vh * sqrtf(fmax_std(0.0f, 1.0f - q1 * q1 - q2 * q2));
@@ -148,7 +155,9 @@ __device__ __forceinline__ bool sample(const Params &p, V3 wo, float u1, float u
     } else {
         const float r = sqrtf(u1);
         const float phi = 2.0f * PI_G * u2;
-        wi = v3(r * cr_cos(phi), r * cr_sin(phi), sqrtf(fmax_std(0.0f, 1.0f - u1)));
+        float sin_phi, cos_phi;
+        cr_sincos(phi, sin_phi, cos_phi);
+        wi = v3(r * cos_phi, r * sin_phi, sqrtf(fmax_std(0.0f, 1.0f - u1)));
     }
     return wi.z > 0.0f;
 }

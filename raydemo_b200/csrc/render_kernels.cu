@@ -264,7 +264,8 @@ __device__ __forceinline__ bool light_term(const LightRec &l, V3 P, V3 N, V3 B, 
     const float z = frac_modf(halton[hi + 0] + rand_offset);
     const float dir = sqrtf(z);
     const float phi = 2 * PI_F * frac_modf(halton[hi + 1] + rand_offset2);
-    const float cos_phi = cr_cos(phi), sin_phi = cr_sin(phi);
+    float sin_phi, cos_phi;
+    cr_sincos(phi, sin_phi, cos_phi);
     const V3 TT = cross(L, B);
     const V3 BB = cross(L, TT);
     const V3 V = (dir * sin_phi) * BB + sqrtf(1.0f - dir) * L + (dir * cos_phi) * TT;
@@ -570,7 +571,8 @@ __device__ F4 shade_hit(const RenderScene &sc, const PassInfo &pi, int rand_inde
             const float u1 = frac_modf(halton[hi + 0] + rand_offset);
             const float u2 = frac_modf(halton[hi + 1] + rand_offset2);
             const float phi = 2 * PI_F * u2;
-            const float cos_phi = cr_cos(phi), sin_phi = cr_sin(phi);
+            float sin_phi, cos_phi;
+            cr_sincos(phi, sin_phi, cos_phi);
             V3 V;
             float weight = 1.0f;
             if ((pi.flags & PASS_OUTPUT_SH) && pi.bounce <= 2) {
@@ -616,7 +618,8 @@ __device__ F4 shade_hit(const RenderScene &sc, const PassInfo &pi, int rand_inde
             const float z = h * frac_modf(halton[hi + 0] + rand_offset);
             const float dir = sqrtf(z);
             const float phi = 2 * PI_F * frac_modf(halton[hi + 1] + rand_offset2);
-            const float cos_phi = cr_cos(phi), sin_phi = cr_sin(phi);
+            float sin_phi, cos_phi;
+            cr_sincos(phi, sin_phi, cos_phi);
             const V3 TT = cross(V, B);
             const V3 BB = cross(V, TT);
             if (dot(V, plane_N) > 0) {
@@ -655,7 +658,8 @@ __device__ F4 shade_hit(const RenderScene &sc, const PassInfo &pi, int rand_inde
             const float temp = sqrtf(1.0f - z * z);
             const int hj = (int)(((uint32_t)(hash_i(hi) + pi.iteration) & (HALTON_SEQ_LEN - 1)) * HALTON_COUNT) + pi.bounce * 2;
             const float phi = halton[hj + 0] * 2 * PI_F;
-            const float cos_phi = cr_cos(phi), sin_phi = cr_sin(phi);
+            float sin_phi, cos_phi;
+            cr_sincos(phi, sin_phi, cos_phi);
             const V3 TT = normalize(cross(V, B));
             const V3 BB = normalize(cross(V, TT));
             V = (temp * sin_phi) * BB + z * V + (temp * cos_phi) * TT;
@@ -748,7 +752,9 @@ __device__ F4 shade_hit(const RenderScene &sc, const PassInfo &pi, int rand_inde
                 const float sin_t = sqrtf(fmax_std(0.0f, 1.0f - cos_t * cos_t));
                 const float phi = 2.0f * PI_F * uc;
                 const ggx::Frame fs = ggx::make_frame(v3(L.n));
-                const V3 wi = ggx::to_world(fs, v3(sin_t * cr_cos(phi), sin_t * cr_sin(phi), cos_t));
+                float sin_phi, cos_phi;
+                cr_sincos(phi, sin_phi, cos_phi);
+                const V3 wi = ggx::to_world(fs, v3(sin_t * cos_phi, sin_t * sin_phi, cos_t));
                 V3 f_cos;
                 float pdf_b;
                 ggx::eval(prm, wo_l, ggx::to_local(fr, wi), f_cos, pdf_b);
