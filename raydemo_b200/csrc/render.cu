@@ -633,11 +633,15 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
         RG_CUDA_TRY(rb->d_geo_best.ensure(std::max<size_t>(total, 1) * sizeof(uint32_t)));
         geo_best = static_cast<uint32_t *>(rb->d_geo_best.p);
     }
+    // short payloads where nothing reads the rest (a frame without bounces keeps
+    // the full ones: its primary rays can be read back, ray_renderer_debug_read)
+    const bool lite = principled_only && !ref_lights && bounces > 0;
+    rb->pay_lite = lite ? total : 0;
     const SceneView &sv = jobs[0].sc.sv;
     auto enqueue_sample = [&](int sample) -> int {
         // primary rays (GeneratePrimaryRays, CoreRef.cpp:427-505)
         RG_CUDA_TRY(cudaMemsetAsync(cnt, 0, 2 * sizeof(uint32_t), st));
-        RG_CUDA_TRY(launch_raygen_jobs(d_jobs, n_jobs, total, sample, rays[0], pay[0], job[0], cnt + 0, st));
+        RG_CUDA_TRY(launch_raygen_jobs(d_jobs, n_jobs, total, sample, rays[0], pay[0], job[0], cnt + 0, lite, st));
         if (ev) RG_CUDA_TRY(cudaEventRecord(ev[1], st));
         tp.count = cnt + 0;
         tp.ray_job = job[0];
@@ -646,7 +650,7 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
             // SampleMeshInTextureSpace (RendererRef.cpp:142-146): rays and hits of the Geo jobs' texels
             RG_CUDA_TRY(cudaMemsetAsync(geo_best, 0xff, (size_t)total * sizeof(uint32_t), st));
             RG_CUDA_TRY(launch_geo_cover(d_jobs, n_jobs, geo_tris, sample, geo_best, st));
-            RG_CUDA_TRY(launch_geo_rays(d_jobs, n_jobs, total, sample, geo_best, rays[0], pay[0], hits, obj, st));
+            RG_CUDA_TRY(launch_geo_rays(d_jobs, n_jobs, total, sample, geo_best, rays[0], pay[0], hits, obj, lite, st));
         }
         if (ev) RG_CUDA_TRY(cudaEventRecord(ev[2], st));
         // shadow rays of the light samples: the persistent kernel in any-hit mode (the hits buffer is free again)
@@ -663,10 +667,10 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
             if (e != cudaSuccess) return e;
             if (adj)
                 e = launch_adjoint_shade(d_jobs, b, rays[in], pay[in], job[in], adj->state[in], hits, obj, cnt + in, total, rays[out], pay[out],
-                                         job[out], adj->state[out], cnt + out, shadow, adj->args, err, st, ref_lights, principled_only);
+                                         job[out], adj->state[out], cnt + out, shadow, adj->args, err, st, ref_lights, lite);
             else
                 e = launch_shade_jobs(d_jobs, sample, b, rays[in], pay[in], job[in], hits, obj, cnt + in, total, rays[out], pay[out], job[out],
-                                      cnt + out, shadow, max_shadow, lights, principled_only, err, ray_stats, st);
+                                      cnt + out, shadow, max_shadow, lights, lite, err, ray_stats, st);
             if (e != cudaSuccess || !(nee || adj || queued)) return e;
             e = launch_trace_closest(sv, shadow.rays, max_shadow, hits, nullptr, err, nullptr, false, st, tps);
             if (e != cudaSuccess) return e;
@@ -683,7 +687,7 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
                 // SortRays_CPU before each bounce (RendererRef.cpp:200-203): the rays move to the other buffer in hash order
                 const int dst = cur ^ 1;
                 RG_CUDA_TRY(launch_loop_sort(d_jobs, (int)jobs.size(), rays[cur], pay[cur], job[cur], cnt + cur, total, rays[dst], pay[dst], job[dst],
-                                             cnt + dst, rb->d_loop_sort.p, st, err));
+                                             cnt + dst, rb->d_loop_sort.p, st, err, lite));
                 cur = dst;
             }
             if (ev) RG_CUDA_TRY(cudaEventRecord(ev[ev_sorted(bounce)], st));
@@ -715,7 +719,7 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     GraphKey key;
     key.add(d_jobs).add(n_jobs).add(total).add(sample0).add(samples).add(sort_mask).add(bounces).add(resolve).add(adj).add(st);
     for (int q = 0; q < 2; q++) key.add(rays[q]).add(pay[q]).add(job[q]);
-    key.add(hits).add(obj).add(cnt).add(shadow.recs).add(shadow.rays).add(shadow.job).add(shadow.terms).add(max_shadow).add(lights).add(rb->d_loop_sort.p).add(nee).add(ref_lights).add(principled_only);
+    key.add(hits).add(obj).add(cnt).add(shadow.recs).add(shadow.rays).add(shadow.job).add(shadow.terms).add(max_shadow).add(lights).add(rb->d_loop_sort.p).add(nee).add(ref_lights).add(lite);
     key.add(sv.nodes).add(sv.leaf_tris).add(sv.inst).add(sv.n_inst).add(tp.persistent).add(tp.refill_min).add(tp.max_depth).add(tp.views);
     key.add(sv.tlas).add(sv.tlas_inst).add(sv.tlas_count).add(tp.tlas).add(tp.block).add(tp.smem_stack).add(tp.one_tri);
     key.add(ev).add(geo_best).add(geo_tris).add(persp);
@@ -1244,6 +1248,20 @@ int ray_renderer_debug_read(ray_renderer *r, int what, void *dst, uint64_t bytes
     const uint64_t size = what == 2 ? (b->p ? HALTON_COUNT * HALTON_SEQ_LEN * sizeof(float) : 0) : b->bytes;
     *out_bytes = size;
     const uint64_t n = std::min<uint64_t>(bytes, size);
+    if (n && what == 1 && r->pay_lite) { // short payloads (render.cuh): the colour, the depth and the pdf, the rest as a path starts
+        const size_t cap = r->pay_lite;
+        std::vector<unsigned char> raw(cap * LITE_PAYLOAD_BYTES);
+        RG_CUDA_TRY(cudaMemcpy(raw.data(), b->p, raw.size(), cudaMemcpyDeviceToHost));
+        std::vector<RayPayload> full(size / sizeof(RayPayload) + 1, RayPayload{});
+        for (size_t i = 0; i < cap && i < full.size(); i++) {
+            memcpy(full[i].c, raw.data() + 16 * i, 12);
+            memcpy(full[i].pad, raw.data() + 16 * i + 12, 4);
+            memcpy(&full[i].ray_depth, raw.data() + 16 * cap + 4 * i, 4);
+            full[i].ior = 1.0f;
+        }
+        memcpy(dst, full.data(), n);
+        return RAY_OK;
+    }
     if (n) RG_CUDA_TRY(cudaMemcpy(dst, b->p, n, cudaMemcpyDeviceToHost));
     return RAY_OK;
 }

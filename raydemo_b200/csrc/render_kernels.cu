@@ -440,7 +440,7 @@ __device__ F4 shade_hit(const RenderScene &sc, const PassInfo &pi, int rand_inde
     }
 
     Derivs der;
-    compute_derivatives(I, t, v3(ray.do_dx), v3(ray.do_dy), v3(ray.dd_dx), v3(ray.dd_dy), v1, v2, v3v, plane_N, der);
+    if (!PONLY) compute_derivatives(I, t, v3(ray.do_dx), v3(ray.do_dy), v3(ray.dd_dx), v3(ray.dd_dy), v1, v2, v3v, plane_N, der);
 
     const int rand_hash = hash_i(rand_index), rand_hash2 = hash_i(rand_hash), rand_hash3 = hash_i(rand_hash2);
     const float rand_offset = construct_float((uint32_t)rand_hash), rand_offset2 = construct_float((uint32_t)rand_hash2),
@@ -795,10 +795,12 @@ __device__ F4 shade_hit(const RenderScene &sc, const PassInfo &pi, int rand_inde
                     nr.p.c[0] = ray.c[0] * wgt.x;
                     nr.p.c[1] = ray.c[1] * wgt.y;
                     nr.p.c[2] = ray.c[2] * wgt.z;
-                    set3(nr.p.do_dx, der.do_dx);
-                    set3(nr.p.do_dy, der.do_dy);
-                    set3(nr.p.dd_dx, der.dd_dx - 2 * (dot_I_pN * der.dndx + der.ddn_dx * plane_N));
-                    set3(nr.p.dd_dy, der.dd_dy - 2 * (dot_I_pN * der.dndy + der.ddn_dy * plane_N));
+                    if (!PONLY) {
+                        set3(nr.p.do_dx, der.do_dx);
+                        set3(nr.p.do_dy, der.do_dy);
+                        set3(nr.p.dd_dx, der.dd_dx - 2 * (dot_I_pN * der.dndx + der.ddn_dx * plane_N));
+                        set3(nr.p.dd_dy, der.dd_dy - 2 * (dot_I_pN * der.dndy + der.ddn_dy * plane_N));
+                    }
                     nr.p.pad[0] = __float_as_uint(pdf); // for the MIS weight where this ray meets a quad light
                     emit = roulette(nr, cant_terminate, urr);
                     if (vg && vg->valid) {
@@ -921,7 +923,7 @@ __device__ __forceinline__ int job_of(const FrameJob *__restrict__ jobs, int n_j
 // Primary rays of every job, one thread per pixel: job-major, row-major in
 // each job's rect. ray_job[i] records the job of ray i.
 __global__ void k_raygen_jobs(const FrameJob *__restrict__ jobs, int n_jobs, uint32_t total, int sample, float4 *__restrict__ rays,
-                              RayPayload *__restrict__ pay, uint32_t *__restrict__ ray_job, uint32_t *__restrict__ count) {
+                              RayPayload *__restrict__ pay, uint32_t *__restrict__ ray_job, uint32_t *__restrict__ count, bool lite) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) *count = total;
     if (i >= total) return;
@@ -942,7 +944,7 @@ __global__ void k_raygen_jobs(const FrameJob *__restrict__ jobs, int n_jobs, uin
     gen_primary(J.cam, J.k, J.fov_k, J.pi.iteration + sample, x, y, J.w, J.h, J.halton, r0, r1, p);
     rays[2ull * i] = r0;
     rays[2ull * i + 1] = r1;
-    pay[i] = p;
+    if (!lite) pay[i] = p;
 }
 
 // ---- Geo (lightmap) cameras: SampleMeshInTextureSpace, CoreRef.cpp:507-603.
@@ -1046,7 +1048,8 @@ __global__ void __launch_bounds__(GEO_BLOCK) k_geo_cover(const FrameJob *__restr
 // (triangle, instance, t = 1, u = w, v = u); an uncovered texel is a miss
 // along d = 0. Both with colour 1 and zero differentials.
 __global__ void k_geo_rays(const FrameJob *__restrict__ jobs, int n_jobs, uint32_t total, int sample, const uint32_t *__restrict__ best,
-                           float4 *__restrict__ rays, RayPayload *__restrict__ pay, float4 *__restrict__ hits, int32_t *__restrict__ obj) {
+                           float4 *__restrict__ rays, RayPayload *__restrict__ pay, float4 *__restrict__ hits, int32_t *__restrict__ obj,
+                           bool lite) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const FrameJob &J = jobs[job_of(jobs, n_jobs, i)];
@@ -1097,7 +1100,7 @@ __global__ void k_geo_rays(const FrameJob *__restrict__ jobs, int n_jobs, uint32
     for (int q = 0; q < 3; q++) pl.do_dx[q] = pl.dd_dx[q] = pl.do_dy[q] = pl.dd_dy[q] = 0.0f;
     pl.ray_depth = 0;
     pl.pad[0] = pl.pad[1] = pl.pad[2] = 0;
-    pay[i] = pl;
+    if (!lite) pay[i] = pl;
     hits[i] = hit;
     obj[i] = ob;
 }
@@ -1107,9 +1110,12 @@ __global__ void k_geo_rays(const FrameJob *__restrict__ jobs, int n_jobs, uint32
 // with alpha 0. A continuation ray is appended where the path goes on and its
 // job traces another bounce. PONLY: every material of every job's scene is
 // RAY_MAT_PRINCIPLED (and no scene has the reference's lights), so the
-// kernel carries none of the other materials' code. LIGHTS: LightMode.
+// kernel carries none of the other materials' code, and its payloads are the
+// short ones. LIGHTS: LightMode. Blocks per SM: 96 registers hold the PONLY form
+// without spills (2.49 ms of the atrium's 4-sample pass on B200 against 2.69 at
+// 4 blocks), 128 the others with a few.
 template <bool PRIMARY, int LIGHTS, bool PONLY = false>
-__global__ void __launch_bounds__(SHADE_BLOCK, LIGHTS == LIGHTS_TRACED ? 3 : 4) k_shade_jobs(const FrameJob *__restrict__ jobs, int sample, int bounce,
+__global__ void __launch_bounds__(SHADE_BLOCK, LIGHTS == LIGHTS_TRACED ? 3 : PONLY ? 5 : 4) k_shade_jobs(const FrameJob *__restrict__ jobs, int sample, int bounce,
                                                             const float4 *__restrict__ rays, const RayPayload *__restrict__ pay,
                                                             const uint32_t *__restrict__ ray_job, const float4 *__restrict__ hits,
                                                             const int32_t *__restrict__ obj, const uint32_t *__restrict__ in_count,
@@ -1139,7 +1145,14 @@ __global__ void __launch_bounds__(SHADE_BLOCK, LIGHTS == LIGHTS_TRACED ? 3 : 4) 
             j = ray_job[i];
             const FrameJob &J = jobs[j];
             const float4 r0 = rays[2ull * i], r1 = rays[2ull * i + 1];
-            const RayPayload p = pay[i];
+            RayPayload p;
+            if (!PONLY) p = pay[i];
+            else if (!PRIMARY) load_lite(pay, max_rays, i, p);
+            else { // as gen_primary (and the Geo cameras) start a path
+                p.c[0] = p.c[1] = p.c[2] = p.ior = 1.0f;
+                p.ray_depth = 0;
+                p.pad[0] = 0;
+            }
             const uint32_t xy = __float_as_uint(r1.w);
             const int x = (int)(xy >> 16), y = (int)(xy & 0xffffu);
             const int index = y * J.w + x;
@@ -1247,7 +1260,8 @@ __global__ void __launch_bounds__(SHADE_BLOCK, LIGHTS == LIGHTS_TRACED ? 3 : 4) 
             if (append && slot < max_rays) {
                 out_rays[2ull * slot] = nr.r0;
                 out_rays[2ull * slot + 1] = nr.r1;
-                out_pay[slot] = nr.p;
+                if (PONLY) store_lite(out_pay, max_rays, slot, nr.p);
+                else out_pay[slot] = nr.p;
                 out_job[slot] = j;
             }
         }
@@ -1546,7 +1560,7 @@ __device__ __forceinline__ void flush_slots(float *s_gr, float *grad_rough, uint
 // REF_LIGHTS: the scene has the reference's point/spot/directional lights
 // (the replayed shading traces their shadow rays again, as the forward did).
 template <bool PRIMARY, bool REF_LIGHTS, bool PONLY = false>
-__global__ void __launch_bounds__(SHADE_BLOCK, 3) k_adjoint_shade(const FrameJob *__restrict__ jobs, int bounce,
+__global__ void __launch_bounds__(SHADE_BLOCK, PONLY ? 4 : 3) k_adjoint_shade(const FrameJob *__restrict__ jobs, int bounce,
                                                                   const float4 *__restrict__ rays, const RayPayload *__restrict__ pay,
                                                                   const uint32_t *__restrict__ ray_job, const AdjState *__restrict__ adj_in,
                                                                   const float4 *__restrict__ hits, const int32_t *__restrict__ obj,
@@ -1582,7 +1596,14 @@ __global__ void __launch_bounds__(SHADE_BLOCK, 3) k_adjoint_shade(const FrameJob
             const FrameJob &J = jobs[j];
             const RenderScene &sc = J.sc;
             const float4 r0 = rays[2ull * i], r1 = rays[2ull * i + 1];
-            const RayPayload p = pay[i];
+            RayPayload p;
+            if (!PONLY) p = pay[i];
+            else if (!PRIMARY) load_lite(pay, max_rays, i, p);
+            else { // as gen_primary (and the Geo cameras) start a path
+                p.c[0] = p.c[1] = p.c[2] = p.ior = 1.0f;
+                p.ray_depth = 0;
+                p.pad[0] = 0;
+            }
             const uint32_t xy = __float_as_uint(r1.w);
             const int x = (int)(xy >> 16), y = (int)(xy & 0xffffu);
             const int index = y * J.w + x;
@@ -1708,7 +1729,8 @@ __global__ void __launch_bounds__(SHADE_BLOCK, 3) k_adjoint_shade(const FrameJob
             if (append && slot < max_rays) {
                 out_rays[2ull * slot] = nr.r0;
                 out_rays[2ull * slot + 1] = nr.r1;
-                out_pay[slot] = nr.p;
+                if (PONLY) store_lite(out_pay, max_rays, slot, nr.p);
+                else out_pay[slot] = nr.p;
                 out_job[slot] = j;
                 adj_out[slot] = out;
                 cont = slot;
@@ -1809,9 +1831,9 @@ cudaError_t launch_halton_table(const uint16_t *perms, int base_iteration, float
 }
 
 cudaError_t launch_raygen_jobs(const FrameJob *jobs, int n_jobs, uint32_t total, int sample, float4 *rays, RayPayload *pay,
-                               uint32_t *ray_job, uint32_t *count, cudaStream_t st) {
+                               uint32_t *ray_job, uint32_t *count, bool lite, cudaStream_t st) {
     if (total == 0) return cudaSuccess;
-    k_raygen_jobs<<<(total + 255) / 256, 256, 0, st>>>(jobs, n_jobs, total, sample, rays, pay, ray_job, count);
+    k_raygen_jobs<<<(total + 255) / 256, 256, 0, st>>>(jobs, n_jobs, total, sample, rays, pay, ray_job, count, lite);
     return cudaGetLastError();
 }
 
@@ -1823,9 +1845,9 @@ cudaError_t launch_geo_cover(const FrameJob *jobs, int n_jobs, uint32_t max_tris
 }
 
 cudaError_t launch_geo_rays(const FrameJob *jobs, int n_jobs, uint32_t total, int sample, const uint32_t *best, float4 *rays, RayPayload *pay,
-                            float4 *hits, int32_t *obj, cudaStream_t st) {
+                            float4 *hits, int32_t *obj, bool lite, cudaStream_t st) {
     if (total == 0) return cudaSuccess;
-    k_geo_rays<<<(total + 255) / 256, 256, 0, st>>>(jobs, n_jobs, total, sample, best, rays, pay, hits, obj);
+    k_geo_rays<<<(total + 255) / 256, 256, 0, st>>>(jobs, n_jobs, total, sample, best, rays, pay, hits, obj, lite);
     return cudaGetLastError();
 }
 
@@ -1842,8 +1864,8 @@ static int resident_blocks(K kernel, int fallback_per_sm) {
 cudaError_t launch_shade_jobs(const FrameJob *jobs, int sample, int bounce, const float4 *rays, const RayPayload *pay, const uint32_t *ray_job,
                               const float4 *hits, const int32_t *obj, const uint32_t *in_count, uint32_t max_rays, float4 *out_rays,
                               RayPayload *out_pay, uint32_t *out_job, uint32_t *out_count, const ShadowQueue &shadow, uint32_t max_shadow,
-                              LightMode lights, bool principled_only, uint32_t *err, unsigned long long *ray_stats, cudaStream_t st) {
-    const bool ponly = principled_only && lights == LIGHTS_NONE;
+                              LightMode lights, bool lite, uint32_t *err, unsigned long long *ray_stats, cudaStream_t st) {
+    const bool ponly = lite; // (with LIGHTS_NONE)
     static int resident[5] = {0, 0, 0, 0, 0};
     int &res = resident[ponly ? 4 : (int)lights];
     if (res == 0)
@@ -1929,8 +1951,8 @@ cudaError_t launch_adjoint_shade(const FrameJob *jobs, int bounce, const float4 
                                  const AdjState *adj_in, const float4 *hits, const int32_t *obj, const uint32_t *in_count, uint32_t max_rays,
                                  float4 *out_rays, RayPayload *out_pay, uint32_t *out_job, AdjState *adj_out, uint32_t *out_count,
                                  const ShadowQueue &shadow, const AdjArgs &args, uint32_t *err, cudaStream_t st, bool ref_lights,
-                                 bool principled_only) {
-    const bool ponly = principled_only && !ref_lights;
+                                 bool lite) {
+    const bool ponly = lite; // (without the reference's lights)
     static int resident[3] = {0, 0, 0};
     if (resident[0] == 0) resident[0] = resident_blocks(k_adjoint_shade<false, false>, 3);
     if (resident[1] == 0) resident[1] = resident_blocks(k_adjoint_shade<false, true>, 3);

@@ -143,7 +143,7 @@ __global__ void k_loop_keys(const FrameJob *__restrict__ jobs, const float4 *__r
 __global__ void k_loop_gather(const float4 *__restrict__ rays, const RayPayload *__restrict__ pay, const uint32_t *__restrict__ ray_job,
                               const uint32_t *__restrict__ perm, const uint32_t *__restrict__ count, uint32_t capacity,
                               float4 *__restrict__ rays_out, RayPayload *__restrict__ pay_out, uint32_t *__restrict__ job_out,
-                              uint32_t *__restrict__ count_out) {
+                              uint32_t *__restrict__ count_out, bool lite) {
     const uint32_t n = min(*count, capacity);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) *count_out = n;
@@ -152,12 +152,18 @@ __global__ void k_loop_gather(const float4 *__restrict__ rays, const RayPayload 
     if (s >= n) return; // cannot happen: the first n positions hold the n valid rays
     rays_out[2ull * i] = rays[2ull * s];
     rays_out[2ull * i + 1] = rays[2ull * s + 1];
+    job_out[i] = ray_job[s];
+    if (lite) {
+        RayPayload p;
+        load_lite(pay, capacity, s, p);
+        store_lite(pay_out, capacity, i, p);
+        return;
+    }
     static_assert(sizeof(RayPayload) % 16 == 0, "payload copied as uint4");
     const uint4 *src = reinterpret_cast<const uint4 *>(pay + s);
     uint4 *dst = reinterpret_cast<uint4 *>(pay_out + i);
 #pragma unroll
     for (int k = 0; k < (int)(sizeof(RayPayload) / 16); k++) dst[k] = src[k];
-    job_out[i] = ray_job[s];
 }
 
 // The render loop's sort keys: the ray hash from this bit up (the job above).
@@ -178,7 +184,7 @@ size_t loop_sort_scratch_bytes(uint64_t capacity, int n_jobs) {
 
 cudaError_t launch_loop_sort(const FrameJob *jobs, int n_jobs, const float4 *rays, const RayPayload *pay, const uint32_t *ray_job,
                              const uint32_t *count, uint32_t capacity, float4 *rays_out, RayPayload *pay_out, uint32_t *job_out,
-                             uint32_t *count_out, void *scratch, cudaStream_t st, uint32_t *err) {
+                             uint32_t *count_out, void *scratch, cudaStream_t st, uint32_t *err, bool lite) {
     if (capacity == 0) return cudaSuccess;
     const int kb = n_jobs > 1 ? 8 : 4;
     char *p = static_cast<char *>(scratch);
@@ -207,7 +213,7 @@ cudaError_t launch_loop_sort(const FrameJob *jobs, int n_jobs, const float4 *ray
     if (e != cudaSuccess) return e;
     e = radix_sort_pairs(keys, perm, capacity, kb, begin, end, rs_scratch, st, count, true, err, true);
     if (e != cudaSuccess) return e;
-    k_loop_gather<<<blocks, 256, 0, st>>>(rays, pay, ray_job, perm, count, capacity, rays_out, pay_out, job_out, count_out);
+    k_loop_gather<<<blocks, 256, 0, st>>>(rays, pay, ray_job, perm, count, capacity, rays_out, pay_out, job_out, count_out, lite);
     return cudaGetLastError();
 }
 
