@@ -1130,8 +1130,8 @@ int ray_scene_last_trace_info(ray_scene *s, ray_trace_info *out) {
         RG_CUDA_TRY(wait_stream(s->info_stream));
         uint32_t err = 0;
         unsigned long long cnt[2] = {0, 0};
-        RG_CUDA_TRY(cudaMemcpy(&err, s->d_err.p, 4, cudaMemcpyDeviceToHost));
-        RG_CUDA_TRY(cudaMemcpy(cnt, s->d_counters.p, 16, cudaMemcpyDeviceToHost));
+        RG_CUDA_TRY(cudaMemcpy(&err, s->trace_words(), 4, cudaMemcpyDeviceToHost));
+        RG_CUDA_TRY(cudaMemcpy(cnt, s->trace_words() + 2, 16, cudaMemcpyDeviceToHost));
         s->last_info.error_flags = err;
         s->last_info.node_visits = cnt[0];
         s->last_info.tri_tests = cnt[1];
@@ -1205,10 +1205,9 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
     int rc = commit(s);
     if (rc != RAY_OK) return rc;
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : s->stream;
-    RG_CUDA_TRY(s->d_err.ensure(4));
-    RG_CUDA_TRY(s->d_counters.ensure(16));
-    RG_CUDA_TRY(cudaMemsetAsync(s->d_err.p, 0, 4, st));
-    RG_CUDA_TRY(cudaMemsetAsync(s->d_counters.p, 0, 16, st));
+    RG_CUDA_TRY(s->d_trace_state.ensure((8 + ray_scene::TRACE_CHUNKS) * sizeof(uint32_t)));
+    uint32_t *words = s->trace_words();
+    RG_CUDA_TRY(cudaMemsetAsync(words, 0, (8 + ray_scene::TRACE_CHUNKS) * sizeof(uint32_t), st));
     const float4 *d_rays = reinterpret_cast<const float4 *>(rays);
     float4 *d_hits = reinterpret_cast<float4 *>(hits);
     int32_t *d_obj = obj;
@@ -1260,7 +1259,6 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
     }
     SceneView sv{static_cast<const WideNode *>(s->d_nodes.p), static_cast<const TriRec *>(s->d_leaf.p),
                  static_cast<const InstanceRec *>(s->d_inst.p), s->n_inst_dev, s->tlas.nodes, s->tlas.order, s->tlas.count};
-    RG_CUDA_TRY(s->d_next_ray.ensure(8)); // a work counter for each of two concurrent traces
     TraceParams tp;
     tp.persistent = s->tuning.kernel >= 2;
     tp.one_tri = s->tuning.kernel == 3;
@@ -1296,7 +1294,6 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
     for (const MeshRec &m : s->meshes) tp.max_depth = std::max(tp.max_depth, m.bvh.depth);
     if (s->tlas.nodes) tp.max_depth += tlas_stack_levels(s->tlas.depth());
     if (s->tuning.deep_stack) tp.max_depth = 0xffffffffu;
-    uint32_t *next_ray = static_cast<uint32_t *>(s->d_next_ray.p);
     // reordered traces: the hash grid of SortRays_CPU over the scene's box (RendererRef.cpp:48-77)
     const bool reorder = s->tuning.reorder != 0;
     float cell[3];
@@ -1305,9 +1302,11 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
     for (size_t c = 0; c + 1 < cut.size(); c++, k++) {
         const uint64_t b = cut[c], m = cut[c + 1] - b;
         // chunk k's trace: on st or `other` in turn, with its own work counter
-        // (the chunk before the previous one, on the same stream, is done with it)
+        // (past the counters: one of the last two, zeroed again once the chunk
+        // before the previous one, on the same stream, is done with it)
         cudaStream_t ts = (k & 1) ? other : st;
-        tp.next_ray = next_ray + (k & 1);
+        tp.next_zeroed = k < (int)ray_scene::TRACE_CHUNKS;
+        tp.next_ray = words + 8 + (tp.next_zeroed ? k : (int)ray_scene::TRACE_CHUNKS - 2 + (k & 1));
         if (mem == RAY_MEM_HOST && m) {
             RG_CUDA_TRY(cudaMemcpyAsync(static_cast<float4 *>(s->d_rays.p) + 2 * b, rays + 8 * b, m * 32, cudaMemcpyHostToDevice, up));
             if (piped) {
@@ -1326,8 +1325,7 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
         }
         if (win.accessPolicyWindow.num_bytes) RG_CUDA_TRY(cudaStreamSetAttribute(ts, cudaStreamAttributeAccessPolicyWindow, &win));
         RG_CUDA_TRY(launch_trace_closest(sv, d_rays + 2 * b, (uint32_t)m, d_hits + b, d_obj ? d_obj + b : nullptr,
-                                         static_cast<uint32_t *>(s->d_err.p), static_cast<unsigned long long *>(s->d_counters.p), s->counting,
-                                         ts, tp));
+                                         words, reinterpret_cast<unsigned long long *>(words + 2), s->counting, ts, tp));
         if (win.accessPolicyWindow.num_bytes) {
             cudaStreamAttrValue off{};
             RG_CUDA_TRY(cudaStreamSetAttribute(ts, cudaStreamAttributeAccessPolicyWindow, &off));
@@ -1352,8 +1350,7 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
         // this call's error word and counters, copied behind its work (another
         // thread's trace of the scene may reset the device words meanwhile)
         if (!s->h_info) RG_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void **>(&s->h_info), 32, cudaHostAllocDefault));
-        RG_CUDA_TRY(cudaMemcpyAsync(s->h_info, s->d_err.p, 4, cudaMemcpyDeviceToHost, st));
-        RG_CUDA_TRY(cudaMemcpyAsync(s->h_info + 2, s->d_counters.p, 16, cudaMemcpyDeviceToHost, st));
+        RG_CUDA_TRY(cudaMemcpyAsync(s->h_info, words, 24, cudaMemcpyDeviceToHost, st));
         // the download of pageable buffers and the wait for the GPU work, without
         // the API lock when this is the outermost entry point of the thread
         const bool release = t_api_depth == 1;

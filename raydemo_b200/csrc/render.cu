@@ -100,7 +100,7 @@ int ensure_ray_buffers(ray_renderer *r, size_t n) {
 
 // Counters, the sample table and its permutations, the stats events.
 int ensure_frame_state(ray_renderer *r) {
-    RG_CUDA_TRY(r->d_counters.ensure(16 * sizeof(uint32_t)));
+    RG_CUDA_TRY(r->d_counters.ensure(ray_renderer::COUNTER_BYTES));
     if (!r->d_perms.p) {
         const std::vector<uint16_t> perms = halton_permutations();
         RG_CUDA_TRY(r->d_perms.ensure(perms.size() * sizeof(uint16_t)));
@@ -571,7 +571,7 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
         return RAY_ERR_INVALID_ARG;
     }
     const uint32_t max_shadow = (uint32_t)(per_ray * total);
-    ShadowQueue shadow{nullptr, nullptr, nullptr, nullptr, nullptr};
+    ShadowQueue shadow{nullptr, nullptr, nullptr, nullptr, nullptr}; // (count: one per shading launch)
     if (nee || adj || queued) {
         const size_t cap = std::max<size_t>(max_shadow, 1);
         if (!adj) RG_CUDA_TRY(rb->d_shadow.ensure(cap * std::max(sizeof(ShadowRec), sizeof(LightVertexRec))));
@@ -588,8 +588,6 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     uint32_t *cnt = static_cast<uint32_t *>(rb->d_counters.p);
     unsigned long long *ray_stats = reinterpret_cast<unsigned long long *>(cnt + 4);
     uint32_t *err = cnt + 3;
-    uint32_t *shadow_cnt = cnt + 8;
-    shadow.count = shadow_cnt;
     float4 *rays[2] = {static_cast<float4 *>(rb->d_rays[0].p), static_cast<float4 *>(rb->d_rays[1].p)};
     RayPayload *pay[2] = {static_cast<RayPayload *>(rb->d_pay[0].p), static_cast<RayPayload *>(rb->d_pay[1].p)};
     uint32_t *job[2] = {static_cast<uint32_t *>(rb->d_job[0].p), static_cast<uint32_t *>(rb->d_job[1].p)};
@@ -616,7 +614,7 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
         tp.one_tri = (TRACE_VARIANTS[trace_var].one & 1) != 0;
         one_any = (TRACE_VARIANTS[trace_var].one & 2) != 0;
     }
-    tp.next_ray = cnt + 2;
+    tp.next_zeroed = true;
     if (n_jobs > 1) { // each ray traced in its job's scene
         tp.views = reinterpret_cast<const uint8_t *>(d_jobs) + offsetof(FrameJob, sc) + offsetof(RenderScene, sv);
         tp.view_stride = (uint32_t)sizeof(FrameJob);
@@ -639,11 +637,20 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     rb->pay_lite = lite ? total : 0;
     const SceneView &sv = jobs[0].sc.sv;
     auto enqueue_sample = [&](int sample) -> int {
+        // every launch's counters are their own and zeroed together, by the caller
+        // for the first sample: a memset each cost the atrium 148 of its 230
+        // launches per pass (0.16 ms of GPU time on B200 and the gaps around them)
+        if (sample != sample0)
+            RG_CUDA_TRY(cudaMemsetAsync(cnt + ray_renderer::COUNTERS_HEAD, 0, ray_renderer::COUNTERS_SAMPLE * sizeof(uint32_t), st));
+        uint32_t *next = cnt + ray_renderer::COUNTERS_HEAD; // the next unused counter
+        static_assert(2 + 5 * (MAX_BOUNCES + 1) <= (int)ray_renderer::COUNTERS_SAMPLE, "per sample: rays; per bounce: sorted rays, rays, "
+                                                                                       "light samples, two work counters");
+        uint32_t *count_in = next++; // of the rays in the current buffer
         // primary rays (GeneratePrimaryRays, CoreRef.cpp:427-505)
-        RG_CUDA_TRY(cudaMemsetAsync(cnt, 0, 2 * sizeof(uint32_t), st));
-        RG_CUDA_TRY(launch_raygen_jobs(d_jobs, n_jobs, total, sample, rays[0], pay[0], job[0], cnt + 0, lite, st));
+        RG_CUDA_TRY(launch_raygen_jobs(d_jobs, n_jobs, total, sample, rays[0], pay[0], job[0], count_in, lite, st));
         if (ev) RG_CUDA_TRY(cudaEventRecord(ev[1], st));
-        tp.count = cnt + 0;
+        tp.count = count_in;
+        tp.next_ray = next++;
         tp.ray_job = job[0];
         if (persp) RG_CUDA_TRY(launch_trace_closest(sv, rays[0], total, hits, obj, err, nullptr, false, st, tp));
         if (geo_tris) {
@@ -657,20 +664,20 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
         TraceParams tps = tp;
         tps.any = true;
         tps.one_tri = one_any;
-        tps.count = shadow_cnt;
         tps.ray_job = shadow.job;
         // shading of the rays in buffer `in` (bounce b), continuation rays to `out`, then the light samples'
         // shadow rays and the colour of the unblocked ones
-        auto shade = [&](int b, int in, int out) -> cudaError_t {
+        auto shade = [&](int b, int in, int out, uint32_t *count_out) -> cudaError_t {
             cudaError_t e = cudaSuccess;
-            if (nee || adj || queued) e = cudaMemsetAsync(shadow_cnt, 0, sizeof(uint32_t), st);
-            if (e != cudaSuccess) return e;
+            shadow.count = next++;
+            tps.count = shadow.count;
+            tps.next_ray = next++;
             if (adj)
-                e = launch_adjoint_shade(d_jobs, b, rays[in], pay[in], job[in], adj->state[in], hits, obj, cnt + in, total, rays[out], pay[out],
-                                         job[out], adj->state[out], cnt + out, shadow, adj->args, err, st, ref_lights, lite);
+                e = launch_adjoint_shade(d_jobs, b, rays[in], pay[in], job[in], adj->state[in], hits, obj, count_in, total, rays[out], pay[out],
+                                         job[out], adj->state[out], count_out, shadow, adj->args, err, st, ref_lights, lite);
             else
-                e = launch_shade_jobs(d_jobs, sample, b, rays[in], pay[in], job[in], hits, obj, cnt + in, total, rays[out], pay[out], job[out],
-                                      cnt + out, shadow, max_shadow, lights, lite, err, ray_stats, st);
+                e = launch_shade_jobs(d_jobs, sample, b, rays[in], pay[in], job[in], hits, obj, count_in, total, rays[out], pay[out], job[out],
+                                      count_out, shadow, max_shadow, lights, lite, err, ray_stats, st);
             if (e != cudaSuccess || !(nee || adj || queued)) return e;
             e = launch_trace_closest(sv, shadow.rays, max_shadow, hits, nullptr, err, nullptr, false, st, tps);
             if (e != cudaSuccess) return e;
@@ -678,7 +685,9 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
             if (queued) return launch_light_apply(d_jobs, sample, b, shadow, hits, max_shadow, err, ray_stats, st);
             return launch_shadow_apply(d_jobs, sample, b, shadow, hits, max_shadow, err, ray_stats, st);
         };
-        RG_CUDA_TRY(shade(2, 0, 1));
+        uint32_t *count_out = next++;
+        RG_CUDA_TRY(shade(2, 0, 1, count_out));
+        count_in = count_out;
         if (ev) RG_CUDA_TRY(cudaEventRecord(ev[3], st));
         // bounces (RendererRef.cpp:183-278); ray counts stay on the device
         int cur = 1;
@@ -686,18 +695,21 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
             if ((sort_mask >> bounce) & 1u) {
                 // SortRays_CPU before each bounce (RendererRef.cpp:200-203): the rays move to the other buffer in hash order
                 const int dst = cur ^ 1;
-                RG_CUDA_TRY(launch_loop_sort(d_jobs, (int)jobs.size(), rays[cur], pay[cur], job[cur], cnt + cur, total, rays[dst], pay[dst], job[dst],
-                                             cnt + dst, rb->d_loop_sort.p, st, err, lite));
+                RG_CUDA_TRY(launch_loop_sort(d_jobs, (int)jobs.size(), rays[cur], pay[cur], job[cur], count_in, total, rays[dst], pay[dst], job[dst],
+                                             next, rb->d_loop_sort.p, st, err, lite));
+                count_in = next++;
                 cur = dst;
             }
             if (ev) RG_CUDA_TRY(cudaEventRecord(ev[ev_sorted(bounce)], st));
             const int nxt = cur ^ 1;
-            RG_CUDA_TRY(cudaMemsetAsync(cnt + nxt, 0, sizeof(uint32_t), st));
-            tp.count = cnt + cur;
+            tp.count = count_in;
+            tp.next_ray = next++;
             tp.ray_job = job[cur];
             RG_CUDA_TRY(launch_trace_closest(sv, rays[cur], total, hits, obj, err, nullptr, false, st, tp));
             if (ev) RG_CUDA_TRY(cudaEventRecord(ev[ev_traced(bounce)], st));
-            RG_CUDA_TRY(shade(bounce + 3, cur, nxt));
+            count_out = next++;
+            RG_CUDA_TRY(shade(bounce + 3, cur, nxt, count_out));
+            count_in = count_out;
             if (ev) RG_CUDA_TRY(cudaEventRecord(ev[ev_shaded(bounce)], st));
             cur = nxt;
         }
@@ -875,9 +887,7 @@ int ray_render(ray_renderer *r, ray_scene *s, ray_region *region) {
         const int kern = plan.kernel;
 
         uint32_t *cnt = static_cast<uint32_t *>(r->d_counters.p);
-        // [0], [1] ray counts of the two buffers, [2] trace / path work counter,
-        // [3] error flags, [4..7] two uint64: rays traced, shadow segments
-        RG_CUDA_TRY(cudaMemsetAsync(cnt, 0, 8 * sizeof(uint32_t), st));
+        RG_CUDA_TRY(cudaMemsetAsync(cnt, 0, ray_renderer::COUNTER_BYTES, st));
         unsigned long long *ray_stats = reinterpret_cast<unsigned long long *>(cnt + 4);
         uint32_t *err = cnt + 3;
         RG_CUDA_TRY(cudaEventRecord(ev[0], st));
@@ -1003,7 +1013,7 @@ int ray_render_batch(ray_renderer *const *renderers, ray_scene *const *scenes, r
                 RG_CUDA_TRY(cudaStreamWaitEvent(st, r->ev_sync, 0));
             }
             uint32_t *cnt = static_cast<uint32_t *>(r0->d_counters.p);
-            RG_CUDA_TRY(cudaMemsetAsync(cnt, 0, 8 * sizeof(uint32_t), st));
+            RG_CUDA_TRY(cudaMemsetAsync(cnt, 0, ray_renderer::COUNTER_BYTES, st));
             if (!jobs.empty()) {
                 RG_CUDA_TRY(r0->d_jobs.ensure(jobs.size() * sizeof(FrameJob)));
                 RG_CUDA_TRY(cudaMemcpyAsync(r0->d_jobs.p, jobs.data(), jobs.size() * sizeof(FrameJob), cudaMemcpyHostToDevice, st));
@@ -1087,7 +1097,7 @@ int ray_render_diff(ray_renderer *r, ray_scene *s, int first_iteration, int samp
         if (rc != RAY_OK) return rc;
         cudaStream_t st = r->stream;
         uint32_t *cnt = static_cast<uint32_t *>(r->d_counters.p);
-        RG_CUDA_TRY(cudaMemsetAsync(cnt, 0, 16 * sizeof(uint32_t), st));
+        RG_CUDA_TRY(cudaMemsetAsync(cnt, 0, ray_renderer::COUNTER_BYTES, st));
         const FrameJob *d_jobs = static_cast<const FrameJob *>(r->d_jobs.p);
         int nb = 0;
         rc = run_wavefront(r, d_jobs, jobs, std::vector<const ray_scene *>(jobs.size(), s), n_pix * (uint32_t)samples, 0, 0u, st, nullptr, nb,
@@ -1151,7 +1161,7 @@ int ray_render_adjoint_color(ray_renderer *r, ray_scene *s, int first_iteration,
         adj.recs = static_cast<AdjShadowRec *>(r->d_adj_shadow.p);
         cudaStream_t st = r->stream;
         uint32_t *cnt = static_cast<uint32_t *>(r->d_counters.p);
-        RG_CUDA_TRY(cudaMemsetAsync(cnt, 0, 16 * sizeof(uint32_t), st));
+        RG_CUDA_TRY(cudaMemsetAsync(cnt, 0, ray_renderer::COUNTER_BYTES, st));
         int nb = 0;
         rc = run_wavefront(r, static_cast<const FrameJob *>(r->d_jobs.p), jobs, std::vector<const ray_scene *>(jobs.size(), s), total, 0, 0u, st,
                            nullptr, nb, false, &adj);

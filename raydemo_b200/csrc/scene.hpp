@@ -159,7 +159,12 @@ struct ray_scene {
     rg::DeviceBuf d_vertices, d_vtx_indices, d_materials, d_textures, d_texels, d_lights, d_area_lights;
 
     // batch-trace staging and diagnostics
-    rg::DeviceBuf d_rays, d_hits, d_obj, d_err, d_counters, d_next_ray;
+    rg::DeviceBuf d_rays, d_hits, d_obj;
+    // a trace call's words, zeroed together: [0] error flags, [2..5] the counting
+    // kernel's totals (two uint64), [8..] a work counter per chunk
+    static constexpr uint32_t TRACE_CHUNKS = 24;
+    rg::DeviceBuf d_trace_state;
+    uint32_t *trace_words() const { return static_cast<uint32_t *>(d_trace_state.p); }
     rg::DeviceBuf d_order[2]; // reordered traces: keys, order and sort scratch of each of two concurrent chunks
     ray_trace_tuning tuning{3, 8, 0, 0, 32, 64, 16, 0, 0, 0};
     bool counting = false;
@@ -196,8 +201,11 @@ struct ray_renderer {
     rg::DeviceBuf d_temp, d_clean, d_final, d_temp_sh, d_clean_sh;
     // wavefront: two ray buffers (trace record + payload, job ids), hits,
     // instance ids, light samples waiting for their shadow rays; counters
-    // [0..1] ray counts, [2] persistent-trace work counter, [3] errors,
-    // [4..7] rays and shadow segments traced (two uint64), [8] light samples
+    // [2] the path kernel's work counter, [3] errors, [4..7] rays and shadow
+    // segments traced (two uint64), [COUNTERS_HEAD ..] the ray, light-sample and
+    // work counters of a sample's launches, one each, zeroed together
+    static constexpr uint32_t COUNTERS_HEAD = 16, COUNTERS_SAMPLE = 64;
+    static constexpr size_t COUNTER_BYTES = (COUNTERS_HEAD + COUNTERS_SAMPLE) * sizeof(uint32_t);
     rg::DeviceBuf d_rays[2], d_pay[2], d_job[2], d_hits, d_obj, d_counters, d_shadow, d_shadow_rays, d_shadow_job, d_shadow_terms;
     uint32_t pay_lite = 0; // the last wavefront's payloads are the short ones, of so many rays (0: the full ones)
     // differentiable form: the samples' sample buffers, the adjoint's per-ray state and light samples

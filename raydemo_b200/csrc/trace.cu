@@ -572,8 +572,10 @@ cudaError_t launch_tuned(const SceneView &sv, const float4 *rays, uint32_t n, fl
         if (e != cudaSuccess) return e;
         blocks = sms * (per_sm > 0 ? per_sm : 1);
     }
-    cudaError_t e = cudaMemsetAsync(tp.next_ray, 0, sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
+    if (!tp.next_zeroed) {
+        const cudaError_t e = cudaMemsetAsync(tp.next_ray, 0, sizeof(uint32_t), st);
+        if (e != cudaSuccess) return e;
+    }
     const uint32_t coop = coop_rays(blocks, BLOCK);
     // few rays, the count known here: no more blocks than give each a warp
     const uint32_t grid = n <= coop ? std::min<uint32_t>(blocks, (n + BLOCK / 32 - 1) / (BLOCK / 32)) : (uint32_t)blocks;
@@ -625,8 +627,10 @@ cudaError_t launch_impl(const SceneView &sv, const float4 *rays, uint32_t n, flo
         if (e != cudaSuccess) return e;
         blocks = sms * (per_sm > 0 ? per_sm : 1);
     }
-    cudaError_t e = cudaMemsetAsync(tp.next_ray, 0, sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
+    if (!tp.next_zeroed) {
+        const cudaError_t e = cudaMemsetAsync(tp.next_ray, 0, sizeof(uint32_t), st);
+        if (e != cudaSuccess) return e;
+    }
     const uint32_t coop = coop_rays(blocks, TRACE_BLOCK);
     // shadow rays and rays of several scenes (no counting variants), with one
     // triangle test per step or a node's triangles at once

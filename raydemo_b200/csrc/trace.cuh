@@ -55,6 +55,7 @@ struct TraceParams {
     // (tlas_stack_levels): sizes the stack
     uint32_t max_depth = 0;
     uint32_t *next_ray = nullptr; // device work counter for the persistent kernel
+    bool next_zeroed = false;     // the caller has zeroed it on this stream (else the launch does)
     const uint32_t *count = nullptr; // device ray count: when set, min(n, *count) rays are traced
     // rays of several scenes (persistent kernel only): ray i is traced in the
     // SceneView at views + ray_job[i] * view_stride, and the sv argument is unused
