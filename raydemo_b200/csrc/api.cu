@@ -1265,7 +1265,7 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
     // last two ramp (a quarter, a half of a chunk) so that the first trace
     // starts early and the last download is short
     std::vector<uint64_t> cut{0};
-    if (piped && n >= 4 * chunk) {
+    if (piped && n + 4096 > 4 * chunk) { // (host_chunk rounds a quarter up)
         const uint64_t q = std::max<uint64_t>(1024, (chunk / 4) & ~uint64_t(1023));
         const uint64_t mid = n - 6 * q, parts = (mid + chunk - 1) / chunk, step = ((mid + parts - 1) / parts + 1023) & ~uint64_t(1023);
         cut.push_back(q);

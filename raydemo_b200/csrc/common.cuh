@@ -70,6 +70,32 @@ static_assert(sizeof(InstanceRec) == 96, "InstanceRec must stay 96 bytes");
 
 constexpr int LEAF_MAX_TRIS = 3;
 
+// Programmatic dependent launch: a kernel launched by launch_dependent may be
+// set up while the kernel before it on the stream still ends; it waits for that
+// kernel's end and its writes in wait_prior, which therefore EVERY thread of
+// every kernel launched this way calls before it touches memory (that way a
+// kernel's end also means the end of all before it). What overlaps is the launch
+// itself: about 2 us on B200. No kernel lets its dependents start earlier
+// (griddepcontrol.launch_dependents): their waiting blocks would keep other
+// streams' kernels off the SMs.
+#ifdef __CUDACC__
+__device__ __forceinline__ void wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#endif
+
 } // namespace rg
 
 // Error helpers for host code.

@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common.cuh"
+
 namespace rg {
 
 constexpr int RS_THREADS = 256;                // one digit per thread
@@ -65,9 +67,12 @@ __device__ __forceinline__ void rs_flush_counts(const uint32_t *s_counts, uint32
 // past it is read or written). vals may hold anything; with vals_identity the
 // input values are taken as 0, 1, 2, ... and vals is only written. key_bytes:
 // 4 or 8. err (may be null): device word that gets SORT_ERR_LOOKBACK.
+// recs_out (may be null): the last pass also copies 32-byte records, recs[v]
+// of the item with value v to the item's sorted place.
 // Returns a CUDA error code; n above RS_MAX_ITEMS is cudaErrorInvalidValue.
 cudaError_t radix_sort_pairs(void *keys, uint32_t *vals, uint64_t n, int key_bytes, int begin_bit, int end_bit, void *scratch,
                              cudaStream_t stream, const uint32_t *n_dev = nullptr, bool vals_identity = false,
-                             uint32_t *err = nullptr, bool counted = false);
+                             uint32_t *err = nullptr, bool counted = false, const float4 *recs = nullptr,
+                             float4 *recs_out = nullptr);
 
 } // namespace rg
