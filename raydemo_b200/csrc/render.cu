@@ -543,7 +543,7 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     if (rc != RAY_OK) return rc;
     if (sort_mask) RG_CUDA_TRY(rb->d_loop_sort.ensure(loop_sort_scratch_bytes(std::max<size_t>(total, 1), (int)jobs.size())));
     // light samples of RAY_MAT_PRINCIPLED vertices wait in d_shadow (count in counter [8])
-    // for their shadow rays; the reference's own lights are traced inside the shading
+    // for their shadow rays, and so do the vertices of the reference's own lights (below)
     bool ref_lights = false, nee = false, principled_only = true;
     uint32_t max_lights = 0;
     for (const FrameJob &J : jobs) {
@@ -560,24 +560,36 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     // scenes with one sun each, 4.7 Mpixel, 4 samples, 6 bounces): shading with
     // the shadow rays traced inside 11.3 ms; queued 4.7 ms of shading, 1.6 of
     // any-hit traces and 0.6 of light sums.
-    const LightMode lights = !ref_lights                                            ? LIGHTS_NONE
-                             : (adj || nee || max_lights > MAX_QUEUED_LIGHTS)       ? LIGHTS_TRACED
-                             : max_lights == 1                                      ? LIGHTS_QUEUED_1
-                                                                                    : LIGHTS_QUEUED;
-    const bool queued = lights >= LIGHTS_QUEUED_1;
-    const uint64_t per_ray = lights == LIGHTS_QUEUED ? max_lights : 1;
-    if (per_ray * total > 0xffffffffull) {
-        set_error("too many light samples in one launch");
-        return RAY_ERR_INVALID_ARG;
+    LightMode lights = !ref_lights                                      ? LIGHTS_NONE
+                       : (adj || nee || max_lights > MAX_QUEUED_LIGHTS) ? LIGHTS_TRACED
+                       : max_lights == 1                                ? LIGHTS_QUEUED_1
+                                                                        : LIGHTS_QUEUED;
+    const uint64_t queue_size = (uint64_t)total * (lights == LIGHTS_QUEUED ? max_lights : 1u);
+    if (lights >= LIGHTS_QUEUED_1) {
+        const size_t cap = std::max<size_t>(queue_size, 1);
+        cudaError_t e = queue_size > 0xffffffffull ? cudaErrorMemoryAllocation : rb->d_shadow.ensure(cap * sizeof(LightVertexRec));
+        if (e == cudaSuccess) e = rb->d_shadow_rays.ensure(cap * 2 * sizeof(float4));
+        if (e == cudaSuccess) e = rb->d_shadow_job.ensure(cap * sizeof(uint32_t));
+        if (e == cudaSuccess) e = rb->d_shadow_terms.ensure(cap * sizeof(float4));
+        if (e == cudaSuccess) e = rb->d_hits.ensure(cap * sizeof(float4));
+        if (e == cudaErrorMemoryAllocation) { // no room for the queue: the lights are traced where they shade
+            cudaGetLastError();
+            lights = LIGHTS_TRACED;
+            for (DeviceBuf *q : {&rb->d_shadow, &rb->d_shadow_rays, &rb->d_shadow_job, &rb->d_shadow_terms}) q->release();
+            rc = ensure_ray_buffers(rb, std::max<size_t>(total, 1));
+            if (rc != RAY_OK) return rc;
+        } else {
+            RG_CUDA_TRY(e);
+        }
     }
-    const uint32_t max_shadow = (uint32_t)(per_ray * total);
+    const bool queued = lights >= LIGHTS_QUEUED_1;
+    const uint32_t max_shadow = queued ? (uint32_t)queue_size : total;
     ShadowQueue shadow{nullptr, nullptr, nullptr, nullptr, nullptr}; // (count: one per shading launch)
     if (nee || adj || queued) {
         const size_t cap = std::max<size_t>(max_shadow, 1);
         if (!adj) RG_CUDA_TRY(rb->d_shadow.ensure(cap * std::max(sizeof(ShadowRec), sizeof(LightVertexRec))));
         RG_CUDA_TRY(rb->d_shadow_rays.ensure(cap * 2 * sizeof(float4)));
         RG_CUDA_TRY(rb->d_shadow_job.ensure(cap * sizeof(uint32_t)));
-        if (queued) RG_CUDA_TRY(rb->d_shadow_terms.ensure(cap * sizeof(float4)));
         RG_CUDA_TRY(rb->d_hits.ensure(cap * sizeof(float4)));
         shadow.recs = adj ? static_cast<void *>(adj->recs) : rb->d_shadow.p;
         shadow.rays = static_cast<float4 *>(rb->d_shadow_rays.p);

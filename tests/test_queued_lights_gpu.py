@@ -77,3 +77,31 @@ def test_batch_of_scenes_with_different_light_counts(cuda_device):
     api.render_batch([r for r, _ in built], [s for _, s in built], [api.RegionContext() for _ in built], 3)
     for (r, _), spec in zip(built, specs):
         assert np.array_equal(r.get_pixels_ref().view(np.uint32), _image(spec, 2)[0].view(np.uint32))
+
+
+def test_no_memory_for_the_queue_traces_the_lights_where_they_shade(cuda_device):
+    """The k-th device allocation of a frame fails, for every k: the frame ends
+    with an error, or (the queue's allocations) with the same image."""
+    from raydemo_b200 import capi
+
+    lib, spec = capi.lib(), _spec(2)
+
+    def frame(k):
+        r, sc = _build(spec)
+        r.set_kernel(1)
+        lib.ray_debug_fail_device_alloc(k)
+        try:
+            r.RenderScene(sc, api.RegionContext())
+        except capi.RayError as e:
+            assert e.code == capi.RAY_ERR_OUT_OF_MEMORY, e
+            return None
+        finally:
+            lib.ray_debug_fail_device_alloc(-1)
+        return r.get_pixels_ref().view(np.uint32)
+
+    want = frame(-1)
+    images = [frame(k) for k in range(240)]
+    failed = [k for k, im in enumerate(images) if im is None]
+    assert failed and failed[-1] < 230
+    assert any(im is not None for im in images[:failed[-1]])  # the queue's
+    assert all(np.array_equal(im, want) for im in images if im is not None)
