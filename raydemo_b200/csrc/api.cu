@@ -70,6 +70,38 @@ cudaError_t bounded_wait(Q query) {
 }
 } // namespace
 
+// Page-locked words for the read-back of a host-buffer trace's flags: slots
+// of one block that stays for the process (4 KiB), taken and returned under
+// the API lock; past its slots, an allocation of its own each.
+namespace {
+constexpr size_t PINNED_SLOT = 64, PINNED_SLOTS = 64;
+char *g_pinned = nullptr;
+uint64_t g_pinned_used = 0; // a bit per slot
+} // namespace
+
+cudaError_t pinned_slot(uint32_t **out) {
+    if (!g_pinned) {
+        const cudaError_t e = cudaHostAlloc(reinterpret_cast<void **>(&g_pinned), PINNED_SLOT * PINNED_SLOTS, cudaHostAllocPortable);
+        if (e != cudaSuccess) {
+            g_pinned = nullptr;
+            return e;
+        }
+    }
+    for (size_t k = 0; k < PINNED_SLOTS; k++)
+        if (!((g_pinned_used >> k) & 1u)) {
+            g_pinned_used |= uint64_t(1) << k;
+            *out = reinterpret_cast<uint32_t *>(g_pinned + k * PINNED_SLOT);
+            return cudaSuccess;
+        }
+    return cudaHostAlloc(reinterpret_cast<void **>(out), PINNED_SLOT, cudaHostAllocDefault);
+}
+
+void release_pinned_slot(uint32_t *p) {
+    const char *c = reinterpret_cast<const char *>(p);
+    if (g_pinned && c >= g_pinned && c < g_pinned + PINNED_SLOT * PINNED_SLOTS) g_pinned_used &= ~(uint64_t(1) << ((c - g_pinned) / PINNED_SLOT));
+    else cudaFreeHost(p);
+}
+
 cudaError_t wait_event(cudaEvent_t e) { return bounded_wait([&] { return cudaEventQuery(e); }); }
 cudaError_t wait_stream(cudaStream_t s) { return bounded_wait([&] { return cudaStreamQuery(s); }); }
 
@@ -276,6 +308,7 @@ int commit(ray_scene *s) {
     if (!s->geom_dirty && !s->inst_dirty) return upload_shading(s);
     if (s->geom_dirty) {
     // 1. build the meshes that have no BVH yet
+    DeviceBuf input; // one mesh's vertices, material words and boxes
     for (MeshRec &m : s->meshes) {
         if (m.built) continue;
         const uint32_t n = m.tris_count;
@@ -284,17 +317,18 @@ int commit(ray_scene *s) {
             m.tris_ref = nullptr;
         }
         if (n) {
-            DeviceBuf verts, mat, aabb;
-            RG_CUDA_TRY(verts.ensure(m.verts.size() * sizeof(float)));
-            RG_CUDA_TRY(mat.ensure(m.mat.size() * sizeof(uint32_t)));
-            RG_CUDA_TRY(aabb.ensure((size_t)n * 6 * sizeof(float)));
+            const size_t verts_b = (m.verts.size() * sizeof(float) + 255) & ~size_t(255);
+            const size_t mat_b = (m.mat.size() * sizeof(uint32_t) + 255) & ~size_t(255);
+            RG_CUDA_TRY(input.ensure(verts_b + mat_b + (size_t)n * 6 * sizeof(float)));
+            float *verts = static_cast<float *>(input.p);
+            uint32_t *mat = reinterpret_cast<uint32_t *>(static_cast<char *>(input.p) + verts_b);
+            float *aabb = reinterpret_cast<float *>(static_cast<char *>(input.p) + verts_b + mat_b);
             RG_CUDA_TRY(device_alloc(reinterpret_cast<void **>(&m.tris_ref), (size_t)n * sizeof(TriRec)));
-            RG_CUDA_TRY(cudaMemcpyAsync(verts.p, m.verts.data(), m.verts.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-            RG_CUDA_TRY(cudaMemcpyAsync(mat.p, m.mat.data(), m.mat.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-            RG_CUDA_TRY(launch_preprocess_tris(static_cast<const float *>(verts.p), static_cast<const uint32_t *>(mat.p), n, m.tris_ref,
-                                               static_cast<float *>(aabb.p), st));
+            RG_CUDA_TRY(cudaMemcpyAsync(verts, m.verts.data(), m.verts.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+            RG_CUDA_TRY(cudaMemcpyAsync(mat, m.mat.data(), m.mat.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+            RG_CUDA_TRY(launch_preprocess_tris(verts, mat, n, m.tris_ref, aabb, st));
             free_mesh_bvh(m.bvh); // what an earlier, failed build of this mesh left
-            const int rc = build_mesh_bvh(m.tris_ref, static_cast<const float *>(aabb.p), n, m.bvh, st);
+            const int rc = build_mesh_bvh(m.tris_ref, aabb, n, m.bvh, st);
             if (rc != RAY_OK) return rc;
             RG_CUDA_TRY(wait_stream(st));
         }
@@ -443,7 +477,7 @@ ray_scene::~ray_scene() {
     for (cudaEvent_t e : pipe_ev)
         if (e) cudaEventDestroy(e);
     for (auto &u : users) cudaEventDestroy(u.second);
-    if (h_info) cudaFreeHost(h_info);
+    if (h_info) release_pinned_slot(h_info);
 }
 
 extern "C" {
@@ -1349,7 +1383,7 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
     if (mem == RAY_MEM_HOST) {
         // this call's error word and counters, copied behind its work (another
         // thread's trace of the scene may reset the device words meanwhile)
-        if (!s->h_info) RG_CUDA_TRY(cudaHostAlloc(reinterpret_cast<void **>(&s->h_info), 32, cudaHostAllocDefault));
+        if (!s->h_info) RG_CUDA_TRY(pinned_slot(&s->h_info));
         RG_CUDA_TRY(cudaMemcpyAsync(s->h_info, words, 24, cudaMemcpyDeviceToHost, st));
         // the download of pageable buffers and the wait for the GPU work, without
         // the API lock when this is the outermost entry point of the thread

@@ -100,6 +100,9 @@ cudaError_t wait_stream_unlocked(cudaStream_t st);
 // api.cu: builds pending BVHs and uploads pending scene data, after the
 // kernels already enqueued that read the arrays it overwrites
 int commit(ray_scene *s);
+// api.cu: 64 page-locked bytes of the host (under the API lock)
+cudaError_t pinned_slot(uint32_t **out);
+void release_pinned_slot(uint32_t *p);
 // api.cu: records that work just enqueued on st reads the scene's device arrays
 cudaError_t note_use(ray_scene *s, cudaStream_t st);
 
