@@ -308,7 +308,7 @@ int commit(ray_scene *s) {
     if (!s->geom_dirty && !s->inst_dirty) return upload_shading(s);
     if (s->geom_dirty) {
     // 1. build the meshes that have no BVH yet
-    DeviceBuf input; // one mesh's vertices, material words and boxes
+    DeviceBuf input, scratch; // one mesh's vertices, material words and boxes; its build's arrays
     for (MeshRec &m : s->meshes) {
         if (m.built) continue;
         const uint32_t n = m.tris_count;
@@ -328,12 +328,14 @@ int commit(ray_scene *s) {
             RG_CUDA_TRY(cudaMemcpyAsync(mat, m.mat.data(), m.mat.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
             RG_CUDA_TRY(launch_preprocess_tris(verts, mat, n, m.tris_ref, aabb, st));
             free_mesh_bvh(m.bvh); // what an earlier, failed build of this mesh left
-            const int rc = build_mesh_bvh(m.tris_ref, aabb, n, m.bvh, st);
+            const int rc = build_mesh_bvh(m.tris_ref, aabb, n, m.bvh, scratch, st);
             if (rc != RAY_OK) return rc;
             RG_CUDA_TRY(wait_stream(st));
         }
         m.built = true;
     }
+    input.release();
+    scratch.release();
     // 2. assemble the scene arrays
     uint64_t nodes = 0, tris = 0;
     for (const MeshRec &m : s->meshes) {

@@ -28,7 +28,9 @@ cudaError_t launch_preprocess_tris(const float *verts, const uint32_t *mat, uint
 // aabb (6 floats each): LBVH over 64-bit Morton keys, greedy collapse to
 // 8-wide nodes, quantised child boxes. Allocates out.nodes / out.leaf_tris.
 // Returns RAY_OK or a RAY_ERR_* code (message through set_error).
-int build_mesh_bvh(const TriRec *tris_ref, const float *aabb, uint32_t n, MeshBvh &out, cudaStream_t st);
+// Its scratch arrays lie in `scratch`, which a commit keeps from mesh to mesh.
+struct DeviceBuf;
+int build_mesh_bvh(const TriRec *tris_ref, const float *aabb, uint32_t n, MeshBvh &out, DeviceBuf &scratch, cudaStream_t st);
 
 // The instance tree: an LBVH over the instances' world boxes (Morton codes
 // of the box centres, the same radix sort, binary radix tree and collapse as

@@ -27,6 +27,7 @@
 #include "../../include/raygpu.h"
 #include "bvh.cuh"
 #include "radix_sort.cuh"
+#include "scene.hpp"
 
 namespace rg {
 namespace {
@@ -595,10 +596,11 @@ cudaError_t dalloc(T **p, size_t count) {
     return device_alloc(reinterpret_cast<void **>(p), std::max<size_t>(count, 1) * sizeof(T));
 }
 
-// Scratch arrays of one build in one allocation, released when the build
-// returns: get() lays them out, alloc() makes them. (An allocation and a free
-// each cost up to half a millisecond; with one per array they were two thirds
-// of the time of adding, committing and dropping a mesh of 131,071 triangles.)
+// Scratch arrays of one build in one allocation: get() lays them out, alloc()
+// places them in `arena`, the caller's, grown where it is too small. (An
+// allocation and a free each cost up to half a millisecond; with one per array
+// they were two thirds of the time of adding, committing and dropping a mesh of
+// 131,071 triangles. A commit keeps one arena for all its meshes.)
 struct TmpAllocs {
     struct Slot {
         void **ptr;
@@ -606,22 +608,15 @@ struct TmpAllocs {
     } slots[20];
     int k = 0;
     size_t bytes = 0;
-    void *base = nullptr;
-    ~TmpAllocs() {
-        if (base) cudaFree(base);
-    }
     template <typename T>
     void get(T **ptr, size_t count) {
         slots[k++] = Slot{reinterpret_cast<void **>(ptr), bytes};
         bytes += (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~size_t(255);
     }
-    cudaError_t alloc() {
-        const cudaError_t e = device_alloc(&base, bytes);
-        if (e != cudaSuccess) {
-            base = nullptr;
-            return e;
-        }
-        for (int i = 0; i < k; i++) *slots[i].ptr = static_cast<char *>(base) + slots[i].offset;
+    cudaError_t alloc(DeviceBuf &arena) {
+        const cudaError_t e = arena.ensure(bytes);
+        if (e != cudaSuccess) return e;
+        for (int i = 0; i < k; i++) *slots[i].ptr = static_cast<char *>(arena.p) + slots[i].offset;
         return cudaSuccess;
     }
 };
@@ -642,7 +637,7 @@ void free_mesh_bvh(MeshBvh &b) {
     b.node_count = b.tri_count = b.depth = 0;
 }
 
-int build_mesh_bvh(const TriRec *tris_ref, const float *aabb, uint32_t n, MeshBvh &out, cudaStream_t st) {
+int build_mesh_bvh(const TriRec *tris_ref, const float *aabb, uint32_t n, MeshBvh &out, DeviceBuf &arena, cudaStream_t st) {
     free_mesh_bvh(out);
     if (n == 0) return RAY_OK;
     if (n > 0x7fffffffu) {
@@ -674,7 +669,7 @@ int build_mesh_bvh(const TriRec *tris_ref, const float *aabb, uint32_t n, MeshBv
     tmp.get(&qa, n);
     tmp.get(&qb, n);
     tmp.get(reinterpret_cast<char **>(&scratch), radix_sort_scratch_bytes(n, 8));
-    RG_CUDA_TRY(tmp.alloc());
+    RG_CUDA_TRY(tmp.alloc(arena));
     const uint32_t init_bounds[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
     RG_CUDA_TRY(cudaMemcpyAsync(bounds, init_bounds, sizeof(init_bounds), cudaMemcpyHostToDevice, st));
     k_bounds<<<std::min<uint32_t>((n + 255) / 256, 1184), 256, 0, st>>>(aabb, n, bounds);
@@ -770,7 +765,8 @@ static int build_inst_topology(uint32_t n, InstTree &t, cudaStream_t st) {
     tmp.get(&qa, n);
     tmp.get(&qb, n);
     tmp.get(&scratch, radix_sort_scratch_bytes(n, 8));
-    RG_CUDA_TRY(tmp.alloc());
+    DeviceBuf arena;
+    RG_CUDA_TRY(tmp.alloc(arena));
     const uint32_t init_bounds[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
     RG_CUDA_TRY(cudaMemcpyAsync(bounds, init_bounds, sizeof(init_bounds), cudaMemcpyHostToDevice, st));
     k_bounds<<<std::min<uint32_t>((n + 255) / 256, 1184), 256, 0, st>>>(t.aabb, n, bounds);
