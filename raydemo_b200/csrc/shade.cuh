@@ -56,7 +56,7 @@ __device__ __forceinline__ float cr_pow(float x, float y) { return __double2floa
 // [-pi/4, pi/4], to x^15 and x^16 (truncation below 2^-54), in FP64, rounded
 // once to FP32. Over every float in [0, 2 pi] (1.09e9) the results equal FP64
 // cos() and sin() rounded once, which reduce twice and for any argument. With
-// cr_pow24 and the Sobol product: the atrium's shading 3.95 -> 3.14 ms per
+// cr_pow24 and the Sobol product: the atrium's shading 3.95 -> 3.2 ms per
 // 4-sample pass on B200.
 __device__ __forceinline__ void cr_sincos(float x, float &sin_x, float &cos_x) {
     const double xd = (double)x;
@@ -90,21 +90,31 @@ __device__ __forceinline__ void cr_sincos(float x, float &sin_x, float &cos_x) {
 
 // x^2.4f for the sRGB decode, x in [0.09, 1.001]: the fifth root of x^2 from a
 // single-precision estimate and one Halley step in FP64 (cubic: 2^-20 becomes
-// 2^-59), times x^2, times x^(2.4f - 2.4) = 1 + 9.5e-8 ln x; rounded once to
-// FP32. The logarithm's 2^-22 enters scaled by 9.5e-8, so the relative error is
-// below 2^-45: of the 29.8M floats in the range 5 round to the neighbour of
-// what FP64 pow() rounded once gives, which takes several times the operations.
+// 2^-59), times x^2, times x^(2.4f - 2.4) = exp(t), t = 9.5e-8 ln x, as 1 + t +
+// t^2/2; rounded once to FP32. ln x = e ln 2 + 2 atanh((m - 1) / (m + 1)), m in
+// [0.75, 1.5), the atanh series to its 11th power: below 2^-29, 2^-52 in t. All
+// 29.8M floats of the range round as FP64 pow() rounded once, which takes
+// several times the operations.
 __device__ __forceinline__ float cr_pow24(float x) {
     const double xd = (double)x, a = xd * xd; // exact
-    const float l = __log2f(x);
-    const float yf = exp2f(0.4f * l);
+    const float yf = exp2f(0.4f * __log2f(x));
     const double y = (double)yf, y2 = y * y, y5 = y2 * y2 * y;
     const double d = fma(2.0, a, 3.0 * y5);
     double rd = (double)__frcp_rn((float)d);
     rd = fma(rd, fma(-d, rd, 1.0), rd);
     const double root = fma(y * (a - y5), rd, y);
     const double p = a * root;
-    return __double2float_rn(fma(p * 6.610366635894253e-08, (double)l, p)); // (2.4f - 2.4) ln 2
+    const int e = (__float_as_int(x) - 0x3F400000) >> 23; // x = m 2^e
+    const float m = __int_as_float(__float_as_int(x) - (e << 23));
+    const double m1 = (double)m + 1.0;
+    double r = (double)__frcp_rn((float)m1);
+    r = fma(r, fma(-m1, r, 1.0), r);
+    const double s = ((double)m - 1.0) * r;
+    const float z = (float)s * (float)s;
+    const float q = z * fmaf(z, fmaf(z, fmaf(z, fmaf(z, 1.0f / 11.0f, 1.0f / 9.0f), 1.0f / 7.0f), 0.2f), 1.0f / 3.0f);
+    const double l = fma(0.6931471805599453, (double)e, 2.0 * fma(s, (double)q, s));
+    const double t = 9.5367431640625005e-08 * l; // 2.4f - 2.4
+    return __double2float_rn(fma(p, fma(0.5 * t, t, t), p));
 }
 
 // std::modf's fractional part: x - trunc(x) is exact for finite x.
