@@ -1,5 +1,6 @@
-// Kernels of the renderer: sample table, primary rays, shading (with shadow
-// rays traced in the kernel), and the accumulate/tone pass. One thread per
+// Kernels of the renderer: sample table, primary rays, shading (its shadow rays
+// appended to a queue or traced in the kernel, LightMode), the sums of the
+// queued lights, and the accumulate/tone pass. One thread per
 // ray or pixel; ray counts live on the device so a frame's bounces run back
 // to back without a host round trip.
 #include "ggx.cuh"
