@@ -547,8 +547,10 @@ __global__ void k_tlas_collapse(const QItem *__restrict__ in, uint32_t n_in, QIt
 // Boxes of the instance tree's nodes [first, first + count), one level, the
 // deeper levels done: from the instances' world boxes and the child nodes'. A
 // node over a box that is not finite (an instance placed by a transform with
-// infinities or NaN) gets an infinite quantum, which leaves all its planes
-// unbounded in the traversal: its instances are left to their own test.
+// infinities or NaN) gets an infinite quantum and zero plane bytes (a refit
+// finds the last boxes' there), which leaves all its planes unbounded in the
+// traversal, the containment test on zero axes included (0 * inf is NaN): its
+// instances are left to their own test.
 __global__ void k_tlas_boxes(uint32_t first, uint32_t count, const float *__restrict__ aabb, const uint32_t *__restrict__ slot_src,
                              float *__restrict__ box, WideNode *__restrict__ nodes) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -580,6 +582,7 @@ __global__ void k_tlas_boxes(uint32_t first, uint32_t count, const float *__rest
         for (int a = 0; a < 3; a++) {
             nd.p[a] = 0.0f;
             nd.e[a] = 255;
+            for (int s = 0; s < 8; s++) nd.qlo[a][s] = nd.qhi[a][s] = 0;
             nlo[a] = -INFINITY;
             nhi[a] = INFINITY;
         }
