@@ -19,6 +19,7 @@
 #include <unordered_set>
 
 #include "../../include/raygpu.h"
+#include "host_chunks.hpp"
 #include "radix_sort.cuh"
 #include "scene.hpp"
 #include "sort.cuh"
@@ -1263,22 +1264,7 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
         if (host_pinned(rays) && host_pinned(hits) && (!obj || host_pinned(obj))) chunk = host_chunk(n);
     }
     const bool piped = chunk < n;
-    // chunk boundaries: with three or more full chunks, the first two and the
-    // last two ramp (a quarter, a half of a chunk) so that the first trace
-    // starts early and the last download is short
-    std::vector<uint64_t> cut{0};
-    if (piped && n + 4096 > 4 * chunk) { // (host_chunk rounds a quarter up)
-        const uint64_t q = std::max<uint64_t>(1024, (chunk / 4) & ~uint64_t(1023));
-        const uint64_t mid = n - 6 * q, parts = (mid + chunk - 1) / chunk, step = ((mid + parts - 1) / parts + 1023) & ~uint64_t(1023);
-        cut.push_back(q);
-        cut.push_back(3 * q);
-        for (uint64_t b = 3 * q + step; b < n - 3 * q; b += step) cut.push_back(b);
-        cut.push_back(n - 3 * q);
-        cut.push_back(n - q);
-    } else {
-        for (uint64_t b = chunk; b < n; b += chunk) cut.push_back(b);
-    }
-    cut.push_back(n);
+    const std::vector<uint64_t> cut = trace_cuts(n, chunk);
     cudaStream_t up = st, down = st, other = st;
     if (piped) {
         for (int k = 0; k < 3; k++)
