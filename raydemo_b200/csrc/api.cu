@@ -126,6 +126,32 @@ void DeviceBuf::release() {
     bytes = 0;
 }
 
+SharedScratch::~SharedScratch() {
+    if (ev) cudaEventDestroy(ev);
+}
+
+cudaError_t ScratchTurn::take(SharedScratch &s, cudaStream_t st) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(st, &cap);
+    if (e != cudaSuccess || cap != cudaStreamCaptureStatusNone) return e;
+    unsigned long long id = 0;
+    e = cudaStreamGetId(st, &id);
+    if (e == cudaSuccess && s.ev && s.last != id) e = cudaStreamWaitEvent(st, s.ev, 0);
+    if (e == cudaSuccess && !s.ev) e = cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+    s.last = id;
+    s_ = &s;
+    st_ = st;
+    return cudaSuccess;
+}
+
+cudaError_t ScratchTurn::end() {
+    if (!s_) return cudaSuccess;
+    const cudaError_t e = cudaEventRecord(s_->ev, st_);
+    s_ = nullptr;
+    return e;
+}
+
 // InverseMatrix, src/Ray/internal/Core.cpp:909-949 (same operation order).
 static void inverse_matrix(const float m[16], float o[16]) {
     const float A2323 = m[10] * m[15] - m[11] * m[14];
@@ -1242,6 +1268,8 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
     int rc = commit(s);
     if (rc != RAY_OK) return rc;
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : s->stream;
+    ScratchTurn turn;
+    RG_CUDA_TRY(turn.take(s->trace_scratch, st));
     RG_CUDA_TRY(s->d_trace_state.ensure((8 + ray_scene::TRACE_CHUNKS) * sizeof(uint32_t)));
     uint32_t *words = s->trace_words();
     RG_CUDA_TRY(cudaMemsetAsync(words, 0, (8 + ray_scene::TRACE_CHUNKS) * sizeof(uint32_t), st));
@@ -1373,6 +1401,7 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
         // thread's trace of the scene may reset the device words meanwhile)
         if (!s->h_info) RG_CUDA_TRY(pinned_slot(&s->h_info));
         RG_CUDA_TRY(cudaMemcpyAsync(s->h_info, words, 24, cudaMemcpyDeviceToHost, st));
+        RG_CUDA_TRY(turn.end()); // (before the API lock goes)
         // the download of pageable buffers and the wait for the GPU work, without
         // the API lock when this is the outermost entry point of the thread
         const bool release = t_api_depth == 1;

@@ -68,6 +68,31 @@ struct DeviceBuf {
     ~DeviceBuf() { release(); }
 };
 
+// Scratch in device memory that calls on several streams share: a call takes
+// its turn before it touches the scratch (its stream waits for the last call's
+// work, if that ran on another stream) and ends it behind its last use; a turn
+// that is not ended ends with its scope. Streams are told apart by their id,
+// which, unlike a handle, is not given out twice. Under stream capture neither
+// waits nor records: there the order is the program's that launches the graph.
+struct SharedScratch {
+    cudaEvent_t ev = nullptr;
+    unsigned long long last = 0; // id of the last call's stream
+    ~SharedScratch();
+};
+class ScratchTurn {
+public:
+    cudaError_t take(SharedScratch &s, cudaStream_t st);
+    cudaError_t end();
+    ScratchTurn() = default;
+    ScratchTurn(const ScratchTurn &) = delete;
+    ScratchTurn &operator=(const ScratchTurn &) = delete;
+    ~ScratchTurn() { end(); }
+
+private:
+    SharedScratch *s_ = nullptr;
+    cudaStream_t st_ = nullptr;
+};
+
 // api.cu: the lock every C-ABI entry point holds while it runs. The entry
 // points only enqueue GPU work (and wait where the call is synchronous), so
 // concurrent calls from several threads -- the reference renders disjoint
@@ -166,6 +191,8 @@ struct ray_scene {
     // a trace call's words, zeroed together: [0] error flags, [2..5] the counting
     // kernel's totals (two uint64), [8..] a work counter per chunk
     static constexpr uint32_t TRACE_CHUNKS = 24;
+    // It and the orders of reordered traces belong to one call at a time.
+    rg::SharedScratch trace_scratch;
     rg::DeviceBuf d_trace_state;
     uint32_t *trace_words() const { return static_cast<uint32_t *>(d_trace_state.p); }
     rg::DeviceBuf d_order[2]; // reordered traces: keys, order and sort scratch of each of two concurrent chunks
