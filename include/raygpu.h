@@ -231,7 +231,9 @@ int ray_scene_commit(ray_scene *s);
  * (CoreRef.cpp:1133-1222). rays: n records of 8 floats
  * (ox, oy, oz, tmax, dx, dy, dz, unused); hits: n ray_hit; obj (optional, may be
  * NULL): n mesh-instance indices (-1 on a miss). mem: RAY_MEM_HOST or
- * RAY_MEM_DEVICE for all three buffers. stream: a cudaStream_t or NULL. */
+ * RAY_MEM_DEVICE for all three buffers. stream: a cudaStream_t or NULL. Calls
+ * on one scene run one after another on the GPU, in the order of the calls,
+ * whatever their streams. */
 int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit *hits, int32_t *obj, int mem, void *stream);
 
 /* ---- ray sorting: SortRays_CPU (CoreRef.cpp:615-657) on device buffers.
@@ -243,7 +245,8 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
  * position k (a stable sort on the hash, the order SortRays_CPU produces);
  * rays_out (may be NULL): the rays in that order. Device memory only;
  * stream-ordered (stream: a cudaStream_t or NULL for the renderer's stream).
- * The sort's scratch memory belongs to the renderer. At most 2^30 - 1 rays. */
+ * The sort's scratch memory belongs to the renderer, whose sorts run one after
+ * another, whatever their streams. At most 2^30 - 1 rays. */
 int ray_sort_rays(ray_renderer *r, const float *rays, uint64_t n, const float root_min[3], const float cell_size[3], uint32_t *keys_out,
                   uint32_t *perm_out, float *rays_out, void *stream);
 

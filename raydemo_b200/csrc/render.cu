@@ -821,8 +821,10 @@ int ray_sort_rays(ray_renderer *r, const float *rays, uint64_t n, const float ro
     }
     if (n == 0) return RAY_OK;
     RG_CUDA_TRY(cudaSetDevice(r->device));
-    RG_CUDA_TRY(r->d_sort_scratch.ensure(sort_rays_scratch_bytes(n)));
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : r->stream;
+    ScratchTurn turn;
+    RG_CUDA_TRY(turn.take(r->sort_scratch, st));
+    RG_CUDA_TRY(r->d_sort_scratch.ensure(sort_rays_scratch_bytes(n)));
     RG_CUDA_TRY(sort_rays(reinterpret_cast<const float4 *>(rays), n, root_min, cell_size, keys_out, perm_out,
                           reinterpret_cast<float4 *>(rays_out), r->d_sort_scratch.p, st));
     return RAY_OK;

@@ -223,7 +223,8 @@ struct ray_renderer {
     ray_stats stats{};
     std::vector<ray_pixel> host_pixels;
     std::vector<ray_shl1> host_sh;
-    rg::DeviceBuf d_sort_scratch, d_loop_sort;
+    rg::DeviceBuf d_sort_scratch, d_loop_sort; // of ray_sort_rays, of the wavefront
+    rg::SharedScratch sort_scratch;            // d_sort_scratch belongs to one call at a time
     rg::DeviceBuf d_geo_best; // Geo cameras: the covering triangle per texel
 
     // framebuffers (w * h): the sample being accumulated, the running mean,
