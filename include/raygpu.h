@@ -344,9 +344,9 @@ int ray_scene_debug_read(ray_scene *s, int what, void *dst, uint64_t bytes, uint
 /* Failure detection (no counterpart in the reference, whose OpenCL backend
  * returns silently on any error, RendererOCL.cpp:474-632), for tests that make
  * failures happen on the host:
- * ray_scene_debug_write overwrites bytes of the committed wide nodes (what 0)
- * or leaf triangles (what 1) from host memory, as a corrupt structure would
- * hold them; the traversal bounds-checks every node and triangle index it
+ * ray_scene_debug_write overwrites bytes of the committed wide nodes (what 0),
+ * leaf triangles (what 1) or instance tree nodes (what 3, 80 bytes each) from
+ * host memory, as a corrupt structure would hold them; the traversal bounds-checks every node and triangle index it
  * reads and bounds its steps, so a trace of such a scene ends every ray and
  * reports RAY_ERR_CUDA (corrupt structure) or RAY_ERR_STACK_OVERFLOW instead
  * of reading out of bounds. Scene edits that rebuild the BVH restore it.

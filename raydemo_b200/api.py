@@ -281,7 +281,7 @@ class Scene:
 
     def debug_write(self, what: int, offset: int, data: bytes) -> None:
         """ray_scene_debug_write: overwrite bytes of the committed wide nodes
-        (0) or leaf triangles (1), for failure-detection tests."""
+        (0), leaf triangles (1) or instance tree nodes (3), for failure-detection tests."""
         b = C.create_string_buffer(bytes(data), len(data))
         check(lib().ray_scene_debug_write(self._h, what, offset, b, len(data)))
 

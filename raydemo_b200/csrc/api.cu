@@ -1470,14 +1470,16 @@ int ray_scene_debug_write(ray_scene *s, int what, uint64_t offset, const void *s
     RG_API_LOCK;
     RG_CHECK(!s || live_scene(s), "unknown or destroyed scene handle");
     RG_CHECK(s && (src || bytes == 0), "null argument");
-    RG_CHECK(what == 0 || what == 1, "invalid array selector");
+    RG_CHECK(what == 0 || what == 1 || what == 3, "invalid array selector");
     RG_GUARD_BEGIN
     RG_CUDA_TRY(cudaSetDevice(s->device));
     const int rc = commit(s);
     if (rc != RAY_OK) return rc;
-    const uint64_t total = what == 0 ? (uint64_t)s->total_nodes * sizeof(WideNode) : (uint64_t)s->total_tris * sizeof(TriRec);
+    const uint64_t total = what == 0   ? (uint64_t)s->total_nodes * sizeof(WideNode)
+                           : what == 1 ? (uint64_t)s->total_tris * sizeof(TriRec)
+                                       : (uint64_t)s->tlas.count * sizeof(WideNode);
     RG_CHECK(offset <= total && bytes <= total - offset, "write outside the array");
-    char *dst = static_cast<char *>(what == 0 ? s->d_nodes.p : s->d_leaf.p);
+    char *dst = static_cast<char *>(what == 0 ? s->d_nodes.p : what == 1 ? s->d_leaf.p : static_cast<void *>(s->tlas.nodes));
     // after the work in flight that reads the scene
     for (auto &u : s->users) RG_CUDA_TRY(cudaStreamWaitEvent(s->stream, u.second, 0));
     if (bytes) RG_CUDA_TRY(cudaMemcpyAsync(dst + offset, src, bytes, cudaMemcpyHostToDevice, s->stream));

@@ -130,10 +130,12 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
     best.prim = -1;
     if constexpr (BEST_SMEM) best.slot = s_best + threadIdx.x;
     // the ray in world space (origin, reciprocals) and the tree's visit count,
-    // kept while the lane is inside an instance
+    // kept while the lane is inside an instance (without room in shared memory
+    // the count in a register, the ray read again)
     constexpr bool WORLD_SMEM = TLAS && (SDEPTH * 8 + 12 + 28) * BLOCK <= 48 * 1024;
     __shared__ float s_world[WORLD_SMEM ? 7 * BLOCK : 1];
     float *world = s_world + (WORLD_SMEM ? threadIdx.x : 0);
+    uint32_t tree_visits = 0;
     LocalRay r = make_local_ray(0.0f, 0.0f, 0.0f, 1.0f, 1.0f, 1.0f);
     MeshRef mr{};
     uint32_t ng_base = 0, ng_bits = 0, tg_base = 0, tg_bits = 0;
@@ -220,6 +222,7 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
         }
         const float4 r0 = __ldg(rays + 2ull * ri), r1 = __ldg(rays + 2ull * ri + 1);
         if (WORLD_SMEM) world[6 * BLOCK] = __uint_as_float(visits);
+        else tree_visits = visits;
         enter(lsv, lsv.inst + m, m, r0, r1);
         in_tree = false;
         sp0 = st.sp;
@@ -235,7 +238,7 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
             } else {
                 const float4 r0 = __ldg(rays + 2ull * ri), r1 = __ldg(rays + 2ull * ri + 1);
                 r = world_ray(r0.x, r0.y, r0.z, safe_inv(r1.x), safe_inv(r1.y), safe_inv(r1.z));
-                visits = 0;
+                visits = tree_visits;
             }
             mr = tree_of(MULTI ? scene_of(ri) : sv);
             in_tree = true;
@@ -364,6 +367,7 @@ __device__ __forceinline__ void trace_persistent(SceneView sv, const float4 *__r
             take(ri);
             take(mi);
             take(visits);
+            if constexpr (TLAS && !WORLD_SMEM) take(tree_visits);
             take(sp0);
             take(st.sp);
             take_flag(in_mesh);
