@@ -542,8 +542,8 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     int rc = ensure_ray_buffers(rb, std::max<size_t>(total, 1));
     if (rc != RAY_OK) return rc;
     if (sort_mask) RG_CUDA_TRY(rb->d_loop_sort.ensure(loop_sort_scratch_bytes(std::max<size_t>(total, 1), (int)jobs.size())));
-    // light samples of RAY_MAT_PRINCIPLED vertices wait in d_shadow (count in counter [8])
-    // for their shadow rays, and so do the vertices of the reference's own lights (below)
+    // light samples of RAY_MAT_PRINCIPLED vertices wait in d_shadow (a counter per shading
+    // launch) for their shadow rays, and so do the vertices of the reference's own lights (below)
     bool ref_lights = false, nee = false, principled_only = true;
     uint32_t max_lights = 0;
     for (const FrameJob &J : jobs) {
@@ -554,20 +554,22 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     }
     // The reference's lights: their shadow rays join the queue for the
     // persistent any-hit trace where every scene has at most MAX_QUEUED_LIGHTS
-    // of them (the queue holds that many rays per ray of the launch, 100 bytes
-    // each) and none has area lights (whose emission the shading adds to the
-    // same colour), else the shading kernel traces them. Measured on B200 (16
+    // of them (the queue holds that many rays per ray of the launch), none has
+    // area lights (whose emission the shading adds to the same colour) and the
+    // queue, which the renderer keeps, stays below MAX_QUEUE_BYTES; else the
+    // shading kernel traces them. Measured on B200 (16
     // scenes with one sun each, 4.7 Mpixel, 4 samples, 6 bounces): shading with
     // the shadow rays traced inside 11.3 ms; queued 4.7 ms of shading, 1.6 of
     // any-hit traces and 0.6 of light sums.
-    LightMode lights = !ref_lights                                      ? LIGHTS_NONE
-                       : (adj || nee || max_lights > MAX_QUEUED_LIGHTS) ? LIGHTS_TRACED
-                       : max_lights == 1                                ? LIGHTS_QUEUED_1
-                                                                        : LIGHTS_QUEUED;
-    const uint64_t queue_size = (uint64_t)total * (lights == LIGHTS_QUEUED ? max_lights : 1u);
+    const uint64_t queue_size = (uint64_t)total * std::max(max_lights, 1u);
+    const bool queueable = !adj && !nee && max_lights <= MAX_QUEUED_LIGHTS && queue_size <= MAX_QUEUE_BYTES / QUEUE_RAY_BYTES;
+    LightMode lights = !ref_lights       ? LIGHTS_NONE
+                       : !queueable      ? LIGHTS_TRACED
+                       : max_lights == 1 ? LIGHTS_QUEUED_1
+                                         : LIGHTS_QUEUED;
     if (lights >= LIGHTS_QUEUED_1) {
         const size_t cap = std::max<size_t>(queue_size, 1);
-        cudaError_t e = queue_size > 0xffffffffull ? cudaErrorMemoryAllocation : rb->d_shadow.ensure(cap * sizeof(LightVertexRec));
+        cudaError_t e = rb->d_shadow.ensure(cap * sizeof(LightVertexRec));
         if (e == cudaSuccess) e = rb->d_shadow_rays.ensure(cap * 2 * sizeof(float4));
         if (e == cudaSuccess) e = rb->d_shadow_job.ensure(cap * sizeof(uint32_t));
         if (e == cudaSuccess) e = rb->d_shadow_terms.ensure(cap * sizeof(float4));

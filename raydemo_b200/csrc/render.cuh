@@ -245,6 +245,11 @@ constexpr uint32_t LIGHT_COUNT_SHIFT = 8;
 // vertex, for the persistent any-hit trace.
 enum LightMode { LIGHTS_NONE = 0, LIGHTS_TRACED = 1, LIGHTS_QUEUED_1 = 2, LIGHTS_QUEUED = 3 };
 constexpr uint32_t MAX_QUEUED_LIGHTS = 4;
+// The queue's memory per shadow ray (record, ray, job, term, hit), and its
+// bound: 9.2 million shadow rays, a 4K frame with one light. A larger frame
+// with several would otherwise hold gigabytes for the renderer's life.
+constexpr uint64_t QUEUE_RAY_BYTES = sizeof(LightVertexRec) + 2 * sizeof(float4) + sizeof(uint32_t) + 2 * sizeof(float4);
+constexpr uint64_t MAX_QUEUE_BYTES = 1ull << 30;
 
 // ---- the path-replay adjoint (differentiable parameters of RAY_MAT_PRINCIPLED)
 constexpr int ADJ_MAX_SLOTS = 64; // roughness slots
