@@ -645,10 +645,11 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
         RG_CUDA_TRY(rb->d_geo_best.ensure(std::max<size_t>(total, 1) * sizeof(uint32_t)));
         geo_best = static_cast<uint32_t *>(rb->d_geo_best.p);
     }
-    // short payloads where nothing reads the rest (a frame without bounces keeps
-    // the full ones: its primary rays can be read back, ray_renderer_debug_read)
-    const bool lite = principled_only && !ref_lights && bounces > 0;
-    rb->pay_lite = lite ? total : 0;
+    // short payloads where nothing reads the rest. The primary rays' are known
+    // to their shading and not written, but for a frame without bounces: its
+    // primary rays can be read back (ray_renderer_debug_read), with full payloads.
+    const bool lite = principled_only && !ref_lights, lite_primary = lite && bounces > 0;
+    rb->pay_lite = lite_primary ? total : 0;
     const SceneView &sv = jobs[0].sc.sv;
     auto enqueue_sample = [&](int sample) -> int {
         // every launch's counters are their own and zeroed together, by the caller
@@ -661,7 +662,7 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
                                                                                        "light samples, two work counters");
         uint32_t *count_in = next++; // of the rays in the current buffer
         // primary rays (GeneratePrimaryRays, CoreRef.cpp:427-505)
-        RG_CUDA_TRY(launch_raygen_jobs(d_jobs, n_jobs, total, sample, rays[0], pay[0], job[0], count_in, lite, st));
+        RG_CUDA_TRY(launch_raygen_jobs(d_jobs, n_jobs, total, sample, rays[0], pay[0], job[0], count_in, lite_primary, st));
         if (ev) RG_CUDA_TRY(cudaEventRecord(ev[1], st));
         tp.count = count_in;
         tp.next_ray = next++;
@@ -671,7 +672,7 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
             // SampleMeshInTextureSpace (RendererRef.cpp:142-146): rays and hits of the Geo jobs' texels
             RG_CUDA_TRY(cudaMemsetAsync(geo_best, 0xff, (size_t)total * sizeof(uint32_t), st));
             RG_CUDA_TRY(launch_geo_cover(d_jobs, n_jobs, geo_tris, sample, geo_best, st));
-            RG_CUDA_TRY(launch_geo_rays(d_jobs, n_jobs, total, sample, geo_best, rays[0], pay[0], hits, obj, lite, st));
+            RG_CUDA_TRY(launch_geo_rays(d_jobs, n_jobs, total, sample, geo_best, rays[0], pay[0], hits, obj, lite_primary, st));
         }
         if (ev) RG_CUDA_TRY(cudaEventRecord(ev[2], st));
         // shadow rays of the light samples: the persistent kernel in any-hit mode (the hits buffer is free again)
