@@ -307,9 +307,11 @@ int ray_scene_last_trace_info(ray_scene *s, ray_trace_info *out);
  * context's persisting-L2 limit, which lasts as long as the context).
  * instance_tree: 0 = traces walk an instance tree (a BVH over the instances'
  * world boxes, built on the GPU at commit, refitted when only transforms
- * changed; the reference's macro tree, SceneRef.cpp:492-516) from 8
- * instances on and test the instance boxes in turn below that; 1 = the tree
- * from 2 instances on; -1 = never. */
+ * changed; the reference's macro tree, SceneRef.cpp:492-516) from 32
+ * instances on and test the instance boxes in turn below that, frames of the
+ * wavefront of 32,768 or more camera rays from 8 instances on (the first one
+ * after a commit builds or refits it); 1 = the tree from 2 instances on; -1 =
+ * never. */
 typedef struct ray_trace_tuning {
     int kernel, refill_min, deep_stack, reorder, reorder_bits, block, smem_stack, stream_hint, l2_persist, instance_tree;
 } ray_trace_tuning;
@@ -324,9 +326,9 @@ typedef struct ray_bvh_info {
 } ray_bvh_info;
 int ray_scene_mesh_bvh_info(ray_scene *s, uint32_t mesh, ray_bvh_info *out);
 
-/* The instance tree after the last commit: instances it covers (0: none,
- * the traversal tests the instance boxes in turn), host milliseconds the
- * last commit spent building or refitting it (device work included), and
+/* The instance tree after the last commit: instances it covers (0: none, or
+ * left to the next frame; the traversal tests the instance boxes in turn),
+ * host milliseconds its last build or refit took (device work included), and
  * whether that was a refit (1) or a build (0). */
 typedef struct ray_instance_tree_info {
     uint32_t instances;

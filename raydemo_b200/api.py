@@ -265,7 +265,7 @@ class Scene:
         1 ray hash, 2 origin cell first), the key bits it sorts on, threads
         per block and shared stack entries (0: 64 and 16), streaming cache
         hint on rays and hits, L2 residency (1 nodes, 2 leaf triangles),
-        instance tree (0 from 8 instances, 1 always, -1 never)."""
+        instance tree (0 from 32 instances, frames from 8; 1 always, -1 never)."""
         t = capi.TraceTuning(kernel, refill_min, deep_stack, reorder, reorder_bits, block, smem_stack, stream_hint, l2_persist,
                              instance_tree)
         check(lib().ray_scene_set_trace_tuning(self._h, C.byref(t)))

@@ -325,6 +325,28 @@ cudaError_t note_use(ray_scene *s, cudaStream_t st) {
     return cudaEventRecord(ev, st);
 }
 
+// The instance tree over the boxes of the last commit, on the scene's stream: a
+// refit when only instances moved (same count, no mesh rebuilt), else a build.
+static int update_inst_tree(ray_scene *s) {
+    const uint32_t ni = (uint32_t)(s->inst_boxes.size() / 6);
+    const bool refit = !s->tlas_rebuild && s->tlas.n == ni;
+    const auto t0 = std::chrono::steady_clock::now();
+    const int rc = build_inst_tree(s->inst_boxes.data(), ni, refit, s->tlas, s->stream);
+    if (rc != RAY_OK) return rc;
+    RG_CUDA_TRY(wait_stream(s->stream));
+    s->last_tlas_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    s->last_tlas_refit = refit ? 1 : 0;
+    s->tlas_stale = s->tlas_rebuild = false;
+    return RAY_OK;
+}
+
+int frame_tree(ray_scene *s, uint64_t rays) {
+    if (!s->tlas_stale || rays < TLAS_MIN_FRAME_RAYS) return RAY_OK;
+    RG_CUDA_TRY(cudaSetDevice(s->device));
+    for (auto &u : s->users) RG_CUDA_TRY(cudaStreamWaitEvent(s->stream, u.second, 0)); // frames in flight read the tree
+    return update_inst_tree(s);
+}
+
 int commit(ray_scene *s) {
     if (!s->geom_dirty && !s->inst_dirty && !s->shade_dirty) return RAY_OK;
     const bool geom_changed = s->geom_dirty;
@@ -399,9 +421,9 @@ int commit(ray_scene *s) {
     s->max_depth = 0;
     for (const MeshRec &m : s->meshes) s->max_depth = std::max(s->max_depth, m.bvh.depth);
     }
-    // 3. instances (SetMeshInstanceTransform, SceneRef.cpp:370-414). The
-    // instance level is a list the traversal tests box by box, so a moved
-    // instance costs this upload of its record and no rebuild.
+    // 3. instances (SetMeshInstanceTransform, SceneRef.cpp:370-414). A moved
+    // instance costs this upload of its record and, where there is an instance
+    // tree, its refit; no mesh is rebuilt.
     const std::vector<uint32_t> &node_base = s->node_base, &tri_base = s->tri_base;
     std::vector<InstanceRec> inst;
     for (const InstanceRecHost &ih : s->instances) {
@@ -430,28 +452,26 @@ int commit(ray_scene *s) {
     if (!inst.empty())
         RG_CUDA_TRY(cudaMemcpyAsync(s->d_inst.p, inst.data(), inst.size() * sizeof(InstanceRec), cudaMemcpyHostToDevice, st));
     s->n_inst_dev = (uint32_t)inst.size();
-    // the instance tree: a refit when only instances moved (same count, no
-    // mesh rebuilt), else a build; none below the tuning's instance count
+    // the instance tree: built here where the traces walk it, else marked for
+    // the first frame that does (frame_tree)
     {
         const uint32_t ni = (uint32_t)inst.size();
         const int mode = s->tuning.instance_tree;
-        const bool want = mode >= 0 && ni >= 2 && (mode == 1 || ni >= TLAS_MIN_INSTANCES);
-        if (!want) {
+        s->tlas_traced = mode >= 0 && ni >= 2 && (mode == 1 || ni >= TLAS_MIN_INSTANCES);
+        s->tlas_stale = s->tlas_traced || (mode >= 0 && ni >= TLAS_MIN_FRAME_INSTANCES);
+        s->tlas_rebuild = s->tlas_rebuild || geom_changed;
+        s->inst_boxes.clear();
+        if (!s->tlas_stale) {
             free_inst_tree(s->tlas);
         } else {
-            std::vector<float> boxes(6 * (size_t)ni);
-            for (size_t i = 0; i < inst.size(); i++)
-                for (int k = 0; k < 3; k++) {
-                    boxes[6 * i + k] = inst[i].bbox_min[k];
-                    boxes[6 * i + 3 + k] = inst[i].bbox_max[k];
-                }
-            const bool refit = !geom_changed && s->tlas.n == ni;
-            const auto t0 = std::chrono::steady_clock::now();
-            const int rc = build_inst_tree(boxes.data(), ni, refit, s->tlas, st);
-            if (rc != RAY_OK) return rc;
-            RG_CUDA_TRY(wait_stream(st));
-            s->last_tlas_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-            s->last_tlas_refit = refit ? 1 : 0;
+            for (const InstanceRec &q : inst) {
+                s->inst_boxes.insert(s->inst_boxes.end(), q.bbox_min, q.bbox_min + 3);
+                s->inst_boxes.insert(s->inst_boxes.end(), q.bbox_max, q.bbox_max + 3);
+            }
+            if (s->tlas_traced) {
+                const int rc = update_inst_tree(s);
+                if (rc != RAY_OK) return rc;
+            }
         }
     }
     // the scene's box: the union of the instance boxes (the ray hash grid of the render loop's sort)
@@ -1132,7 +1152,7 @@ int ray_scene_instance_tree_info(ray_scene *s, ray_instance_tree_info *out) {
     RG_GUARD_BEGIN
     const int rc = commit(s);
     if (rc != RAY_OK) return rc;
-    out->instances = s->tlas.nodes ? s->tlas.n : 0;
+    out->instances = s->tlas.nodes && !s->tlas_stale ? s->tlas.n : 0;
     out->refit = s->last_tlas_refit;
     out->ms = s->last_tlas_ms;
     return RAY_OK;
@@ -1307,8 +1327,7 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
         RG_CUDA_TRY(cudaStreamWaitEvent(up, s->pipe_ev[0], 0));
         RG_CUDA_TRY(cudaStreamWaitEvent(other, s->pipe_ev[0], 0));
     }
-    SceneView sv{static_cast<const WideNode *>(s->d_nodes.p), static_cast<const TriRec *>(s->d_leaf.p),
-                 static_cast<const InstanceRec *>(s->d_inst.p), s->n_inst_dev, s->tlas.nodes, s->tlas.order, s->tlas.count};
+    const SceneView sv = scene_view(s, s->tlas_traced);
     TraceParams tp;
     tp.persistent = s->tuning.kernel >= 2;
     tp.one_tri = s->tuning.kernel == 3;
@@ -1316,7 +1335,7 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
     tp.block = s->tuning.block;
     tp.smem_stack = s->tuning.smem_stack;
     tp.stream_hint = s->tuning.stream_hint;
-    tp.tlas = s->tlas.nodes != nullptr;
+    tp.tlas = sv.tlas != nullptr;
     // L2 residency of the nodes or leaf triangles: an access-policy window on
     // the streams the traces run on, taken off again once they are enqueued
     cudaStreamAttrValue win{};
@@ -1342,7 +1361,7 @@ int ray_scene_trace_closest(ray_scene *s, const float *rays, uint64_t n, ray_hit
         }
     }
     for (const MeshRec &m : s->meshes) tp.max_depth = std::max(tp.max_depth, m.bvh.depth);
-    if (s->tlas.nodes) tp.max_depth += tlas_stack_levels(s->tlas.depth());
+    if (sv.tlas) tp.max_depth += tlas_stack_levels(s->tlas.depth());
     if (s->tuning.deep_stack) tp.max_depth = 0xffffffffu;
     // reordered traces: the hash grid of SortRays_CPU over the scene's box (RendererRef.cpp:48-77)
     const bool reorder = s->tuning.reorder != 0;

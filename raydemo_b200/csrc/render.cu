@@ -614,9 +614,10 @@ int run_wavefront(ray_renderer *rb, const FrameJob *d_jobs, const std::vector<Fr
     tp.refill_min = scn[0]->tuning.refill_min;
     for (int j = 0; j < n_jobs; j++) {
         bounces = std::max(bounces, jobs[j].bounces);
-        const uint32_t levels = scn[j]->max_depth + (scn[j]->tlas.nodes ? tlas_stack_levels(scn[j]->tlas.depth()) : 0u);
+        const bool tree = jobs[j].sc.sv.tlas != nullptr;
+        const uint32_t levels = scn[j]->max_depth + (tree ? tlas_stack_levels(scn[j]->tlas.depth()) : 0u);
         tp.max_depth = std::max(tp.max_depth, scn[j]->tuning.deep_stack ? 0xffffffffu : levels);
-        if (scn[j]->tlas.nodes) tp.tlas = true; // the kernels that can walk an instance tree
+        if (tree) tp.tlas = true; // the kernels that can walk an instance tree
     }
     tp.block = scn[0]->tuning.block;
     tp.smem_stack = scn[0]->tuning.smem_stack;
@@ -779,6 +780,9 @@ int diff_jobs(ray_renderer *r, ray_scene *s, int first_iteration, int samples, s
         set_error("too many pixels x samples");
         return RAY_ERR_INVALID_ARG;
     }
+    rc = frame_tree(s, (uint64_t)n_pix * samples);
+    if (rc != RAY_OK) return rc;
+    J.sc.sv = scene_view(s, true);
     RG_CUDA_TRY(r->d_diff_temp.ensure((size_t)n_pix * samples * sizeof(float4)));
     jobs.assign(samples, J);
     for (int k = 0; k < samples; k++) {
@@ -903,6 +907,12 @@ int ray_render(ray_renderer *r, ray_scene *s, ray_region *region) {
             plan_frame(r, s, s->total_tris, (uint32_t)(s->lights.size() + s->area_lights.size()), (uint32_t)n_pix, J.bounces, J.geo.on != 0);
         const int kern = plan.kernel;
 
+        if (kern != 2) { // (the path kernel tests the instances in turn)
+            rc = frame_tree(s, n_pix);
+            if (rc != RAY_OK) return rc;
+            J.sc.sv = scene_view(s, true);
+        }
+
         uint32_t *cnt = static_cast<uint32_t *>(r->d_counters.p);
         RG_CUDA_TRY(cudaMemsetAsync(cnt, 0, ray_renderer::COUNTER_BYTES, st));
         unsigned long long *ray_stats = reinterpret_cast<unsigned long long *>(cnt + 4);
@@ -1005,6 +1015,7 @@ int ray_render_batch(ray_renderer *const *renderers, ray_scene *const *scenes, r
             for (int i = 0; i < count; i++) run = std::min(run, HALTON_SEQ_LEN - ((regions[i]->iteration + 1) & (HALTON_SEQ_LEN - 1)));
             std::vector<FrameJob> jobs;
             std::vector<const ray_scene *> jscn;
+            std::vector<ray_scene *> trees; // of the jobs
             jobs.reserve(count);
             uint64_t total = 0;
             for (int i = 0; i < count; i++) {
@@ -1021,7 +1032,14 @@ int ray_render_batch(ray_renderer *const *renderers, ray_scene *const *scenes, r
                 }
                 jobs.push_back(J);
                 jscn.push_back(scenes[i]);
+                trees.push_back(scenes[i]);
             }
+            if (kern != 2)
+                for (size_t j = 0; j < jobs.size(); j++) {
+                    rc = frame_tree(trees[j], total);
+                    if (rc != RAY_OK) return rc;
+                    jobs[j].sc.sv = scene_view(trees[j], true);
+                }
             // the batch runs on the first renderer's stream, after each renderer's own work
             for (int i = 0; i < count; i++) {
                 ray_renderer *r = renderers[i];

@@ -125,6 +125,9 @@ cudaError_t wait_stream_unlocked(cudaStream_t st);
 // api.cu: builds pending BVHs and uploads pending scene data, after the
 // kernels already enqueued that read the arrays it overwrites
 int commit(ray_scene *s);
+// api.cu: before a launch of frames over `rays` camera rays: brings the scene's
+// instance tree up to date where such launches walk it and the commit left it
+int frame_tree(ray_scene *s, uint64_t rays);
 // api.cu: 64 page-locked bytes of the host (under the API lock)
 cudaError_t pinned_slot(uint32_t **out);
 void release_pinned_slot(uint32_t *p);
@@ -136,6 +139,7 @@ int add_texture(ray_scene *s, const uint8_t *data, int w, int h, bool srgb, bool
 void compute_tangent_basis(std::vector<VertexRec> &vertices, std::vector<uint32_t> &indices, size_t vtx_start);
 int upload_shading(ray_scene *s); // device copies of vertices, materials, textures and lights
 RenderScene render_scene_view(const ray_scene *s);
+SceneView scene_view(const ray_scene *s, bool tree); // tree: with the instance tree, if it is up to date
 
 // A cached CUDA graph of a launch sequence (render.cu: graph_run).
 struct GraphSlot {
@@ -181,8 +185,13 @@ struct ray_scene {
     // device arrays assembled at commit
     rg::DeviceBuf d_nodes, d_leaf, d_inst, d_tris_ref;
     uint32_t n_inst_dev = 0;
-    rg::InstTree tlas;               // the instance tree (built at commit from TLAS_MIN_INSTANCES instances)
-    double last_tlas_ms = 0.0;       // host time of the last commit's instance-tree build or refit
+    // the instance tree: built at commit where batch traces walk it (tlas_traced),
+    // else by the first frame that does (tlas_stale: not up to date)
+    rg::InstTree tlas;
+    bool tlas_traced = false, tlas_stale = false;
+    bool tlas_rebuild = false;       // meshes changed since it was built: no refit
+    std::vector<float> inst_boxes;   // the instances' world boxes (6 floats each) of the last commit, where there is a tree
+    double last_tlas_ms = 0.0;       // host time of the last instance-tree build or refit
     int last_tlas_refit = 0;         // 1: it was a refit
     rg::DeviceBuf d_vertices, d_vtx_indices, d_materials, d_textures, d_texels, d_lights, d_area_lights;
 

@@ -340,10 +340,20 @@ int upload_shading(ray_scene *s) {
     return RAY_OK;
 }
 
+SceneView scene_view(const ray_scene *s, bool tree) {
+    SceneView v{static_cast<const WideNode *>(s->d_nodes.p), static_cast<const TriRec *>(s->d_leaf.p),
+                static_cast<const InstanceRec *>(s->d_inst.p), s->n_inst_dev};
+    if (tree && !s->tlas_stale) {
+        v.tlas = s->tlas.nodes;
+        v.tlas_inst = s->tlas.order;
+        v.tlas_count = s->tlas.count;
+    }
+    return v;
+}
+
 RenderScene render_scene_view(const ray_scene *s) {
     RenderScene r{};
-    r.sv = SceneView{static_cast<const WideNode *>(s->d_nodes.p), static_cast<const TriRec *>(s->d_leaf.p),
-                     static_cast<const InstanceRec *>(s->d_inst.p), s->n_inst_dev, s->tlas.nodes, s->tlas.order, s->tlas.count};
+    r.sv = scene_view(s, true);
     r.tris = static_cast<const TriRec *>(s->d_tris_ref.p);
     r.vtx_indices = static_cast<const uint32_t *>(s->d_vtx_indices.p);
     r.vertices = static_cast<const VertexRec *>(s->d_vertices.p);

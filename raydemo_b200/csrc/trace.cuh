@@ -19,11 +19,18 @@ struct SceneView {
     uint32_t tlas_count = 0;
 };
 
-// Instance counts from which traces walk the instance tree instead of
-// testing every instance box in turn: one wide node holds 8 boxes. Measured
-// on B200 (1M incoherent rays, spheres of 1,280 triangles, in turn / tree):
-// 4 instances 271 / 290 us, 8 314 / 307, 16 442 / 342, 64 1348 / 507.
-constexpr uint32_t TLAS_MIN_INSTANCES = 8;
+// Instance counts from which launches walk the instance tree instead of
+// testing every instance box in turn (one wide node holds 8 boxes). Batch
+// traces, measured on B200 (us per pass, spheres of 320 triangles, one moved
+// before each pass / none moved; tree against in turn): 16 instances, 500 rays
+// 81 / 45 against 53 / 41, 100,000 rays 150 / 115 against 128 / 119; 31
+// instances, 500 rays 108 / 86 against 74 / 74, 1M rays 458 / 433 against 489 /
+// 478: below 32 the refit costs more than it gives. Frames trace the same
+// tree many times over (the atrium, 17 instances, 8 bounces: 128 x 128 pixels
+// 0.98 against 0.99 ms, 256 x 256 1.30 against 1.43, 1280 x 720 3.38 against
+// 3.84; a refit is 0.03).
+constexpr uint32_t TLAS_MIN_INSTANCES = 32, TLAS_MIN_FRAME_INSTANCES = 8;
+constexpr uint64_t TLAS_MIN_FRAME_RAYS = 32768;
 // Stack entries a ray holds at most beside its mesh's while it traverses an
 // instance of a tree of the given depth: a group per tree level, and the
 // rest of the leaf group it came from.
