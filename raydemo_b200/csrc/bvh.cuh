@@ -28,7 +28,7 @@ cudaError_t launch_preprocess_tris(const float *verts, const uint32_t *mat, uint
 // aabb (6 floats each): LBVH over 64-bit Morton keys, greedy collapse to
 // 8-wide nodes, quantised child boxes. Allocates out.nodes / out.leaf_tris.
 // Returns RAY_OK or a RAY_ERR_* code (message through set_error).
-// Its scratch arrays lie in `scratch`, which a commit keeps from mesh to mesh.
+// Its scratch arrays lie in `scratch`, which is kept from mesh to mesh.
 struct DeviceBuf;
 int build_mesh_bvh(const TriRec *tris_ref, const float *aabb, uint32_t n, MeshBvh &out, DeviceBuf &scratch, cudaStream_t st);
 

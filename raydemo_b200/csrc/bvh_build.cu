@@ -603,7 +603,7 @@ cudaError_t dalloc(T **p, size_t count) {
 // places them in `arena`, the caller's, grown where it is too small. (An
 // allocation and a free each cost up to half a millisecond; with one per array
 // they were two thirds of the time of adding, committing and dropping a mesh of
-// 131,071 triangles. A commit keeps one arena for all its meshes.)
+// 131,071 triangles. The arena is kept from mesh to mesh and commit to commit.)
 struct TmpAllocs {
     struct Slot {
         void **ptr;
