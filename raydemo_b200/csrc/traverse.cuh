@@ -345,7 +345,8 @@ __device__ __forceinline__ bool node_step(const MeshRef &mr, const LocalRay &r, 
     // a zero direction component leaves its axis' planes NaN, that is unbounded:
     // without this a ray parallel to an axis plane entered every node its
     // other two axes allow, thousands of them, and one such ray among the 4M of
-    // a launch decided the launch's time (5.4 to 14 ms against 3.2 ms on B200)
+    // a launch decided the launch's time (5.4 ms with one seed's rays and 14 with
+    // another's, against 3.2 without such a ray, on B200)
     const uint32_t keep = r.oct > 7u ? zero_axis_children(mr.nodes + ni, r.oct, r.ox, r.oy, r.oz) : 0xFFu;
     const uint4 *np = reinterpret_cast<const uint4 *>(mr.nodes + ni);
     const uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
